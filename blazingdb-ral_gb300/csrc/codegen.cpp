@@ -1877,57 +1877,198 @@ GeneratedKernel generate_filter_kernel(const FilterSpec& f, const Shape& s, bool
 }
 
 // ---- delimited-text scan fused with its filter ---------------------------------------------
-// One warp per chunk of 32 J lines (ticket order).  Pass 1: lane t of slice j takes line
-// base + 32 j + t, finds its fields, parses the predicate's and evaluates the predicate (a blank
-// or skipped line keeps nothing); the slice's keep bits are one ballot word.  The warp looks back
-// for the chunk's output offset, turns the words into the kept-line list and, 32 kept lines per
-// step, parses every projected field of line list[k] in lane k and stores it at offset + k; each
-// output's validity bits of the step are one ballot, OR-ed in at the step's bit offset.
+// Two generated kernels: one finds the lines, evaluates the condition and lists the kept lines, the
+// other parses the projected fields of the listed lines.  Field rules and the staged text's readers:
+// csrc/textscan.cuh.
 extern "C" const char* const ral_textscan_source;
 
-GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s) {
-    if (s.J < 1 || s.J > 32) throw std::runtime_error("text scan kernel shape: J out of range");
-    GeneratedKernel gk;
-    gk.shape = s;
-    ParamLayout& L = gk.layout;
+namespace {
+
+// What the two text scan kernels share: parameter slots, the fields each reads and their identity.
+struct TextScanParts {
+    ParamLayout L;
+    std::vector<int> f1, f2;  // sorted distinct file columns: the condition's, the projections'
+    std::vector<bool> pred_ref, pred_raw;
+    std::string key;
+};
+
+TextScanParts text_scan_parts(const TextScanSpec& t) {
+    TextScanParts r;
     const int NP = (int)t.dtypes.size();
     int slot = kTextScanFixedSlots;
-    L.n_rows = 0;
-    L.out_data = slot; slot += NP;
-    L.out_valid = slot; slot += NP;
-    L.scratch = slot++;
+    r.L.n_rows = 0;
+    r.L.out_data = slot; slot += NP;
+    r.L.out_valid = slot; slot += NP;
+    r.L.scratch = slot++;
     const Program* pred = t.predicate;
     if (pred) {
-        assign_scalar_slots(*pred, L, slot);
-    }
-    L.total = slot;
-
-    // the file fields each pass needs: pass 1 the predicate's, pass 2 every projection's
-    std::vector<bool> pred_ref = pred ? pred->inputs_referenced() : std::vector<bool>();
-    std::vector<bool> pred_raw = pred ? pred->inputs_raw_valid() : std::vector<bool>();
-    std::vector<int> f1, f2;  // sorted distinct file columns
-    if (pred)
+        assign_scalar_slots(*pred, r.L, slot);
+        r.pred_ref = pred->inputs_referenced();
+        r.pred_raw = pred->inputs_raw_valid();
         for (size_t c = 0; c < t.predicate_cols.size(); c++)
-            if (pred_ref[c] || pred_raw[c]) f1.push_back(t.file_cols[t.predicate_cols[c]]);
-    for (int q = 0; q < NP; q++) f2.push_back(t.file_cols[q]);
-    auto uniq = [](std::vector<int>& v) {
-        std::sort(v.begin(), v.end());
-        v.erase(std::unique(v.begin(), v.end()), v.end());
-    };
-    uniq(f1);
-    uniq(f2);
-    auto slot_of = [](const std::vector<int>& v, int fc) {
-        return (int)(std::lower_bound(v.begin(), v.end(), fc) - v.begin());
-    };
-
+            if (r.pred_ref[c] || r.pred_raw[c]) r.f1.push_back(t.file_cols[t.predicate_cols[c]]);
+    }
+    r.L.total = slot;
+    for (int q = 0; q < NP; q++) r.f2.push_back(t.file_cols[q]);
+    for (std::vector<int>* v : {&r.f1, &r.f2}) {
+        std::sort(v->begin(), v->end());
+        v->erase(std::unique(v->begin(), v->end()), v->end());
+    }
     std::ostringstream key;
-    key << "textscan|";
     for (int q = 0; q < NP; q++) key << (int)t.dtypes[q] << "@" << t.file_cols[q] << ",";
     if (pred) {
         key << "|P" << pred->structure_key() << "@";
         for (int c : t.predicate_cols) key << c << ",";
     }
-    key << "|J" << s.J << "T" << s.threads << "B" << s.min_blocks;
+    r.key = key.str();
+    return r;
+}
+
+int text_slot_of(const std::vector<int>& v, int fc) {
+    return (int)(std::lower_bound(v.begin(), v.end(), fc) - v.begin());
+}
+
+// Field finders: the bounds of each needed field (an empty one, or fs = -1, where the line is shorter).
+// The staged line [s, e) walks its delimiter bits, a line that is not staged its bytes in global memory.
+void emit_text_finders(std::ostream& os, const std::vector<int>& fields) {
+    const int last = fields.back();
+    auto needed = [&](int f) { return std::binary_search(fields.begin(), fields.end(), f); };
+    auto at = [&](int f) { return (int)(std::lower_bound(fields.begin(), fields.end(), f) - fields.begin()); };
+    // by steps of one delimiter, whatever lies between them
+    os << "static __device__ __noinline__ ral_u32 ral_nth(const ral_u32* db, ral_u32 s, ral_u32 e, int k) {\n"
+          "    ral_u32 w = s >> 5, bits = db[w & RAL_DBM] & (0xffffffffu << (s & 31u));\n"
+          "    for (;; --k) {\n"
+          "        while (bits == 0u && ((w + 1u) << 5) < e) { ++w; bits = db[w & RAL_DBM]; }\n"
+          "        if (bits == 0u) return ~0u;\n"
+          "        if (k == 0) return (w << 5) + (ral_u32)__ffs((int)bits) - 1u;\n"
+          "        bits &= bits - 1u;\n    }\n}\n";
+    // The first 96 bytes' delimiters in three words; delimiter k's position is d<k> (~0: none found).
+    os << "RAL_FI void ral_fields(const ral_u32* db, ral_u32 s, ral_u32 e, ral_u32* fs, ral_u32* fe) {\n";
+    os << "    const ral_u32 w = s >> 5, sh = s & 31u;\n";
+    os << "    const ral_u32 a1 = db[(w + 1u) & RAL_DBM], a2 = db[(w + 2u) & RAL_DBM];\n";
+    os << "    ral_u32 b0 = __funnelshift_r(db[w & RAL_DBM], a1, sh), b1 = __funnelshift_r(a1, a2, sh);\n";
+    os << "    ral_u32 b2 = __funnelshift_r(a2, db[(w + 3u) & RAL_DBM], sh), at = s - 1u;\n";
+    os << "    // a word without delimiters before one with some\n";
+    os << "    const bool hole = (b0 == 0u && (b1 | b2) != 0u) || (b1 == 0u && b2 != 0u);\n";
+    for (int f = 0; f <= last; f++) {
+        os << "    if (b0 == 0u) { b0 = b1; b1 = b2; b2 = 0u; at += 32u; }\n";
+        if (needed(f) || needed(f + 1)) os << "    ral_u32 d" << f << " = b0 ? at + (ral_u32)__ffs((int)b0) : ~0u;\n";
+        if (f < last) os << "    b0 &= b0 - 1u;\n";
+    }
+    os << "    if (hole || (d" << last << " == ~0u && e - s > 96u)) {\n";
+    for (int f = 0; f <= last; f++)
+        if (needed(f) || needed(f + 1)) os << "        d" << f << " = ral_nth(db, s, e, " << f << ");\n";
+    os << "    }\n";
+    // a field the line does not reach is empty
+    for (int f = 0; f <= last; f++) {
+        if (!needed(f)) continue;
+        if (f == 0) os << "    fs[" << at(f) << "] = s;\n";
+        else os << "    fs[" << at(f) << "] = d" << f - 1 << " < e ? d" << f - 1 << " + 1u : e;\n";
+        os << "    fe[" << at(f) << "] = d" << f << " < e ? d" << f << " : e;\n";
+    }
+    os << "}\n";
+    os << "RAL_FI void ral_fields_slow(const char* d, ral_i64 e, char delim, ral_i64* fs, ral_i64* fe) {\n";
+    os << "#pragma unroll\n    for (int k = 0; k < " << fields.size() << "; ++k) { fs[k] = -1; fe[k] = -1; }\n";
+    os << "    int f = 0;\n    ral_i64 p0 = 0;\n";
+    os << "    for (ral_i64 p = 0;; ++p) {\n";
+    os << "        const bool end = p >= e;\n";
+    os << "        if (end || d[p] == delim) {\n";
+    os << "            switch (f) {\n";
+    for (size_t k = 0; k < fields.size(); k++)
+        os << "            case " << fields[k] << ": fs[" << k << "] = p0; fe[" << k << "] = p; break;\n";
+    os << "            default: break;\n            }\n";
+    os << "            if (end || f >= " << fields.back() << ") break;\n";
+    os << "            ++f;\n            p0 = p + 1;\n";
+    os << "        }\n    }\n}\n";
+}
+
+// The parse of field k into the register value v (the column value widened) and the validity word vw;
+// `refused` counts refusals.  staged: from the view (tx, position fs of a line that starts at s and,
+// in global memory, at ls), else from the line's bytes in global memory.
+void emit_text_parse(std::ostream& os, const std::string& ind, gdf_dtype dt, const std::string& k, const std::string& v,
+                     const std::string& vw, bool staged) {
+    const bool isf = dt == GDF_FLOAT32 || dt == GDF_FLOAT64;
+    const bool date = dt == GDF_DATE32 || dt == GDF_DATE64;
+    const std::string with_time = date ? (dt == GDF_DATE64 ? ", true" : ", false") : "";
+    const std::string what = isf ? "double" : date ? "date" : "int";
+    const std::string fs = "fs[" + k + "]", fe = "fe[" + k + "]";
+    os << ind << "{\n" << ind << "    " << (isf ? "double" : "long long") << " t = 0;\n";
+    if (staged) {
+        os << ind << "    bool ok = ral_txv_" << what << "<RAL_TXM>(tx, " << fs << ", " << fe << with_time << ", &t) & (" << fs
+           << " < " << fe << ");\n";
+        os << ind << "    if (!ok && " << fs << " < " << fe << ") {\n";
+        os << ind << "        const ral_tx_result r = ral_txv_slow_" << what << "(ls + (" << fs << " - s), " << fe << " - " << fs
+           << with_time << ");\n";
+    } else {
+        os << ind << "    bool ok = false;\n" << ind << "    if (" << fs << " >= 0) {\n";
+        os << ind << "        const ral_tx_result r = ral_txv_slow_" << what << "(ls + " << fs << ", " << fe << " - " << fs
+           << with_time << ");\n";
+    }
+    os << ind << "        t = " << (isf ? "__longlong_as_double(r.v)" : "r.v") << ";\n";
+    os << ind << "        ok = r.st == RAL_TX_OK;\n";
+    os << ind << "        if (r.st == RAL_TX_REFUSED) ++refused;\n" << ind << "    }\n";
+    os << ind << "    " << vw << " = ok ? 0xffffffffu : 0u;\n";
+    std::string val = "t";
+    switch (dt) {
+    case GDF_INT8: val = "(ral_i64)(signed char)t"; break;
+    case GDF_INT16: val = "(ral_i64)(short)t"; break;
+    case GDF_INT32: case GDF_DATE32: val = "(ral_i64)(int)t"; break;
+    case GDF_FLOAT32: val = "(double)(float)t"; break;
+    default: break;
+    }
+    os << ind << "    " << v << " = ok ? " << val << " : " << (isf ? "0.0" : "0") << ";\n";
+    os << ind << "}\n";
+}
+
+// Column c's variables around a call of the out-of-line line parser: what it writes through references
+// are copies, so that the columns themselves stay in registers.
+void text_slow_vars(const std::string& c, bool isf, std::string& vars, std::string& call, std::string& copy) {
+    vars += (isf ? "double y" : "ral_i64 y") + c + " = 0; ral_u32 v" + c + " = 0u; ";
+    call += ", y" + c + ", v" + c;
+    copy += "x" + c + " = y" + c + "; w" + c + " = v" + c + "; ";
+}
+
+// Parameters both kernels start with.
+void emit_text_params(std::ostream& os, bool delims) {
+    os << "    const char* const A = (const char*)P.s[1];\n";      // the text's address rounded down to 16
+    os << "    const ral_i64 lo = (ral_i64)P.s[3];\n";             // the text is [lo, hi) of it
+    os << "    const ral_i64 hi = (ral_i64)P.s[2];\n";
+    os << "    ral_u64* const list = (ral_u64*)P.s[4];\n";
+    os << "    const char term = (char)(P.s[6] >> 8);\n";
+    if (delims)
+        os << "    const ral_u32 D4 = (ral_u32)(P.s[6] & 0xffu) * 0x01010101u;\n";
+    os << "    const ral_u64 cap = (ral_u64)P.s[7];\n";
+    os << "    const int lane = threadIdx.x & 31;\n    const int warp = threadIdx.x >> 5;\n";
+}
+
+}  // namespace
+
+// The first of the two kernels of a text scan: every line of the text is found, its condition
+// evaluated, and the kept ones written to a list in text order (start | length << 48; 65535 stands for
+// any longer length).
+//
+// A warp takes a range of RB bytes by ticket and owns the lines that start in it.  It reads the range
+// 1024 bytes at a time, 32 consecutive bytes a lane, the next step's loads in flight; a step leaves
+// the bytes and one bit per delimiter in a ring in shared memory and the terminators' positions in a
+// queue.  Whenever 32 lines are queued (or the oldest would leave the ring) each lane takes one of them:
+// it finds its fields from the delimiter bits and reads them four bytes at a time (ral_txv_*).  The kept
+// lines' count goes through the look-back while the warp scans its next range; their positions wait in
+// shared memory, or, where a range keeps more of them than fit, the range is read a second time.
+//
+// Bound: instruction issue (70% of the slots), about 1060 instructions per 32 lines for TPC-H Q6's three
+// fields and conditions, 510 of them for finding the lines.  The text is read once and no line index is
+// written: 4M lines of 62 bytes take 157 us (1.6 TB/s of text), against 650 us for the form before (a line
+// index of three kernels, 185 us, then a walk of every line byte by byte, 467 us).
+GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s) {
+    GeneratedKernel gk;
+    gk.shape = s;
+    const TextScanParts parts = text_scan_parts(t);
+    gk.layout = parts.L;
+    const ParamLayout& L = gk.layout;
+    const int NP = (int)t.dtypes.size();
+    const Program* pred = t.predicate;
+    std::ostringstream key;
+    key << "textscan|" << parts.key << "|T" << s.threads << "B" << s.min_blocks;
     char hex[32];
     snprintf(hex, sizeof hex, "%016llx", (unsigned long long)fnv1a(key.str()));
     gk.name = std::string("ral_textscan_") + hex;
@@ -1936,8 +2077,9 @@ GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s)
     std::ostringstream os;
     os << ral_textscan_source << "\n";
     os << "// generated: " << key.str() << "\n";
-    os << "#define RAL_J " << s.J << "\n#define RAL_THREADS " << s.threads << "\n";
-    os << "#define RAL_WARPS (RAL_THREADS / 32)\n";
+    os << "#define RAL_THREADS " << s.threads << "\n#define RAL_WARPS (RAL_THREADS / 32)\n";
+    os << "#define RAL_RING 4096u\n#define RAL_QM 511u\n#define RAL_KL " << kTextScanKeptLines << "u\n";
+    os << "#define RAL_TXM (RAL_RING / 4u - 1u)\n#define RAL_DBM (RAL_RING / 32u - 1u)\n";
     os << "struct RalParams { ral_u64 s[" << L.total << "]; };\n\n";
     std::vector<Kind> pred_kind;
     if (pred) {
@@ -1947,231 +2089,426 @@ GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s)
         ValidEmitter ve(*pred);
         ve.emit(os, "    ", [&](int c) { return "fv[" + std::to_string(c) + "]"; });
         os << "    return " << ve.name[pred->final_pos[0]] << ";\n}\n";
-    }
-    os << "RAL_FI void ral_text_line(const char* d, const ral_i64* ends, ral_i64 nterm, ral_i64 nb, ral_i64 i,\n"
-          "                          ral_i64& s, ral_i64& e) {\n"
-          "    s = i == 0 ? 0 : ends[i - 1] + 1;\n"
-          "    e = i < nterm ? ends[i] : nb;\n"
-          "    if (e > s && d[e - 1] == '\\r') --e;\n"
-          "}\n";
-    // The text [S, E) of up to 32 lines copied into the warp's stage by all lanes (16-byte loads
-    // where the text allows, never past its end), so that the lanes' byte-by-byte parsing reads
-    // shared memory instead of 32 lines' worth of global addresses per instruction.  Returns the
-    // pointer through which text position p reads its staged copy, or the text itself when the
-    // span does not fit.
-    os << "#define RAL_STAGE 4096\n";
-    os << "RAL_FI const char* ral_text_stage(const char* d, ral_i64 nb, ral_i64 S, ral_i64 E, char* stage, int lane) {\n"
-          "    const ral_i64 a = S & ~15ll;\n"
-          "    if (E <= S || E - a > RAL_STAGE) return d;\n"
-          "    __syncwarp();\n"
-          "    if ((((unsigned long long)d) & 15ull) == 0ull) {\n"
-          "        for (ral_i64 o = a + 16 * lane; o < E; o += 512) {\n"
-          "            if (o + 16 <= nb) {\n"
-          "                *reinterpret_cast<uint4*>(stage + (o - a)) = __ldcs(reinterpret_cast<const uint4*>(d + o));\n"
-          "            } else {\n"
-          "                for (ral_i64 k = o; k < nb; ++k) stage[k - a] = d[k];\n"
-          "            }\n"
-          "        }\n"
-          "    } else {\n"
-          "        for (ral_i64 o = a + lane; o < E; o += 32) stage[o - a] = d[o];\n"
-          "    }\n"
-          "    __syncwarp();\n"
-          "    return stage - a;\n"
-          "}\n";
-    // field finders: the bounds of each needed field of a line (-1 where the line is shorter)
-    auto finder = [&](const char* name, const std::vector<int>& fields) {
-        os << "RAL_FI void " << name << "(const char* d, ral_i64 s, ral_i64 e, char delim, ral_i64* fs, ral_i64* fe) {\n";
-        os << "#pragma unroll\n    for (int k = 0; k < " << fields.size() << "; ++k) { fs[k] = -1; fe[k] = -1; }\n";
-        os << "    int f = 0;\n    ral_i64 p0 = s;\n";
-        os << "    for (ral_i64 p = s;; ++p) {\n";
-        os << "        const bool end = p >= e;\n";
-        os << "        if (end || d[p] == delim) {\n";
-        os << "            switch (f) {\n";
-        for (size_t k = 0; k < fields.size(); k++)
-            os << "            case " << fields[k] << ": fs[" << k << "] = p0; fe[" << k << "] = p; break;\n";
-        os << "            default: break;\n            }\n";
-        os << "            if (end || f >= " << fields.back() << ") break;\n";
-        os << "            ++f;\n            p0 = p + 1;\n";
-        os << "        }\n    }\n}\n";
-    };
-    if (!f1.empty()) finder("ral_fields_pred", f1);
-    finder("ral_fields_all", f2);
-    // parse of one field into a register value (column value widened) and a validity word
-    // (a refusal is counted where `counts` holds: idle lanes of pass 2 parse a kept line twice)
-    auto parse = [&](const std::string& ind, gdf_dtype dt, const std::string& k, const std::string& v,
-                     const std::string& vw, const std::string& counts) {
-        const bool isf = dt == GDF_FLOAT32 || dt == GDF_FLOAT64;
-        os << ind << (isf ? "double " : "ral_i64 ") << v << " = 0;\n";
-        os << ind << "ral_u32 " << vw << " = 0u;\n";
-        os << ind << "if (fs[" << k << "] >= 0) {\n";
-        if (isf) os << ind << "    double t = 0.0;\n" << ind << "    const int st = ral_tx_parse_double(ds, fs[" << k << "], fe[" << k << "], &t);\n";
-        else if (dt == GDF_DATE32 || dt == GDF_DATE64)
-            os << ind << "    long long t = 0;\n" << ind << "    const int st = ral_tx_parse_date(ds, fs[" << k << "], fe[" << k
-               << "], " << (dt == GDF_DATE64 ? "true" : "false") << ", &t);\n";
-        else os << ind << "    long long t = 0;\n" << ind << "    const int st = ral_tx_parse_int(ds, fs[" << k << "], fe[" << k << "], &t);\n";
-        os << ind << "    if (st == RAL_TX_REFUSED && " << counts << ") ++refused;\n";
-        os << ind << "    if (st == RAL_TX_OK) {\n";
-        os << ind << "        " << vw << " = 0xffffffffu;\n";
-        switch (dt) {
-        case GDF_INT8: os << ind << "        " << v << " = (ral_i64)(signed char)t;\n"; break;
-        case GDF_INT16: os << ind << "        " << v << " = (ral_i64)(short)t;\n"; break;
-        case GDF_INT32: case GDF_DATE32: os << ind << "        " << v << " = (ral_i64)(int)t;\n"; break;
-        case GDF_FLOAT32: os << ind << "        " << v << " = (double)(float)t;\n"; break;
-        default: os << ind << "        " << v << " = t;\n"; break;
+        if (!parts.f1.empty()) emit_text_finders(os, parts.f1);
+        // the condition of a staged line, and of a line in global memory (out of line; refusals come back
+        // above the result's lowest bit)
+        for (const bool staged : {true, false}) {
+            if (staged)
+                os << "RAL_FI bool ral_keep(const RalParams& P, const ral_u32* tx, const ral_u32* db, ral_u32 s, ral_u32 e,\n"
+                      "                     const char* ls, ral_u32& refused) {\n";
+            else
+                os << "static __device__ __noinline__ ral_u32 ral_keep_long(const RalParams& P, const char* ls, ral_i64 n, char delim) {\n"
+                      "    ral_u32 refused = 0u;\n";
+            const char* w = staged ? "ral_u32" : "ral_i64";
+            if (!parts.f1.empty()) {
+                os << "    " << w << " fs[" << parts.f1.size() << "], fe[" << parts.f1.size() << "];\n";
+                os << (staged ? "    ral_fields(db, s, e, fs, fe);\n" : "    ral_fields_slow(ls, n, delim, fs, fe);\n");
+            }
+            os << "    ral_u32 fv[" << std::max<size_t>(1, t.predicate_cols.size()) << "];\n";
+            for (size_t c = 0; c < t.predicate_cols.size(); c++) {
+                if (!(parts.pred_ref[c] || parts.pred_raw[c])) {
+                    os << "    fv[" << c << "] = 0xffffffffu;\n";
+                    continue;
+                }
+                const gdf_dtype dt = t.dtypes[t.predicate_cols[c]];
+                const std::string k = std::to_string(c);
+                os << "    " << (dt == GDF_FLOAT32 || dt == GDF_FLOAT64 ? "double x" : "ral_i64 x") << k << " = 0;\n    ral_u32 w" << k
+                   << " = 0u;\n";
+                emit_text_parse(os, "    ", dt, std::to_string(text_slot_of(parts.f1, t.file_cols[t.predicate_cols[c]])), "x" + k,
+                                "w" + k, staged);
+                os << "    fv[" << k << "] = w" << k << ";\n";
+            }
+            os << "    " << kind_ctype(pred_kind[0]) << " y0;\n    ral_pred_row(P";
+            for (size_t c = 0; c < t.predicate_cols.size(); c++)
+                if (parts.pred_ref[c]) os << ", x" << c;
+            for (size_t c = 0; c < t.predicate_cols.size(); c++)
+                if (parts.pred_raw[c]) os << ", w" << c << " & 1u";
+            os << ", y0);\n";
+            os << "    const bool keep = (ral_pred_vrow(fv) & 1u) != 0u && " << narrow("y0", pred_kind[0], GDF_INT8) << " != 0;\n";
+            os << (staged ? "    return keep;\n}\n" : "    return (keep ? 1u : 0u) | refused << 1;\n}\n");
         }
-        os << ind << "    }\n" << ind << "}\n";
-    };
-
+    }
+    const bool delims = pred && !parts.f1.empty();  // the delimiter bits are only read for fields
+    // a warp's shared memory: the ring's bytes and delimiter bits, two ranges' kept lines (start | length
+    // << 16), the queue, and the 16-byte granules at the text's ends (zero outside it)
+    os << "struct RalWarp {\n    __align__(16) ral_u32 tx[RAL_RING / 4];\n"
+       << (delims ? "    ral_u32 db[RAL_RING / 32];\n" : "") << "    uint4 edge[3];\n    ral_u32 kl[2][RAL_KL];\n    unsigned short q[RAL_QM + 1];\n};\n";
     os << "\nextern \"C\" __global__ void __launch_bounds__(RAL_THREADS, " << std::max(1, s.min_blocks) << ") " << gk.name
        << "(const __grid_constant__ RalParams P) {\n";
-    os << "    __shared__ ral_u32 s_kp[RAL_WARPS][32];\n";
-    os << "    __shared__ unsigned short s_ls[RAL_WARPS][32 * RAL_J];\n";
-    os << "    __shared__ __align__(16) char s_tx[RAL_WARPS][RAL_STAGE];\n";
-    os << "    const ral_i64 T = (ral_i64)P.s[0];\n";
-    os << "    const char* const d = (const char*)P.s[1];\n";
-    os << "    const ral_i64 nb = (ral_i64)P.s[2];\n";
-    os << "    const ral_i64* const ends = (const ral_i64*)P.s[3];\n";
-    os << "    const ral_i64 nterm = (ral_i64)P.s[4];\n";
-    os << "    const ral_i64 skip = (ral_i64)P.s[5];\n";
-    os << "    const char delim = (char)P.s[6];\n";
-    os << "    const ral_u64 cap = (ral_u64)P.s[7];\n";
-    os << "    const ral_u64 obase = (ral_u64)P.s[8];\n";
+    os << "    __shared__ RalWarp s_w[RAL_WARPS];\n";
+    emit_text_params(os, delims);
+    os << "    const ral_i64 nranges = (ral_i64)P.s[0];\n";
+    os << "    const ral_u32 RB = (ral_u32)P.s[5];\n";
+    os << "    const ral_u32 T4 = (ral_u32)(P.s[6] >> 8) * 0x01010101u;\n";
     os << "    ral_u64* const scratch = (ral_u64*)P.s[" << L.scratch << "];\n";
     os << "    ral_u64* const status = scratch + " << text_scan_header(NP) << ";\n";
+    os << "    const ral_i64 start = lo + (ral_i64)scratch[" << text_scan_header(NP) - 1 << "];\n";
+    os << "    RalWarp& W = s_w[warp];\n    ral_u32* const tx = W.tx;\n    unsigned short* const q = W.q;\n";
+    os << R"RALK(    const ral_u32 l32 = 32u * lane, below = (1u << lane) - 1u;
+    ral_u32 refused = 0, over = 0;
+    // Two ranges in flight: range A, scanned and its count published, waits while the warp scans range B,
+    // so that A's predecessors have published by the time its offset is looked up.
+    ral_i64 rangeA = -1;
+    ral_u32 totalA = 0, buf = 0;
+    auto write_list = [&](ral_i64 r, ral_u32 n, const ral_u32* kl) {
+        const ral_u64 excl = ral_lookback_published(status, r, n, scratch + 1);
+        if (r == nranges - 1 && lane == 0) scratch[2] = excl + n;
+        if (lane == 0 && excl + n > cap) ++over;
+        __syncwarp();
+        if (n <= RAL_KL)
+            for (ral_u32 i = lane; i < n; i += 32u) {
+                const ral_u32 w = kl[i];
+                if (excl + i < cap) list[excl + i] = (ral_u64)(r * RB + (w & 0xffffu)) | (ral_u64)(w >> 16) << 48;
+            }
+        return excl;
+    };
+    for (;;) {
+        ral_u32 ticket = 0;
+        if (lane == 0) ticket = atomicAdd((unsigned int*)scratch, 1u);
+        const ral_i64 range = __shfl_sync(0xffffffffu, ticket, 0);
+        if (range >= nranges) break;
+        const ral_i64 base = range * RB;
+        // positions in the range are 32-bit offsets from base (the text's ends clamped to them)
+        const char* const R = A + base;
+        const ral_u32 lo_r = lo > base ? (ral_u32)(lo - base < RB ? lo - base : RB) : 0u;
+        const ral_u32 hi_r = hi > base ? (ral_u32)(hi - base < (1 << 20) ? hi - base : 1 << 20) : 0u;
+        const ral_u32 first = start > base ? (ral_u32)(start - base < RB ? start - base : RB) : 0u;
+        const bool any_line = first < RB && first < hi_r;
+        // no step of this range (nor the one loaded ahead) reaches the text's ends
+        const bool inner = lo_r == 0u && first == 0u && hi_r >= RB + RAL_RING + 2048u;
+        ral_u64 excl = 0;
+        // once; a second time, writing the list as it goes, where the range keeps more lines than W.kl holds
+        for (int pass = 0;; ++pass) {
+            ral_u32 total = 0;
+            if (any_line) {
+                ral_i64 last_end = -1;  // where a line longer than the ring ends
+                // the queue: the position before the first line's start, then terminators; line j lies between
+                // entries j and j + 1 (16 bits: -1 wraps and comes back; 0xffff as an end is last_end)
+                ral_u32 qh = 0, qt = 0;
+                __syncwarp();
+                if (base + first == start || R[(ral_i64)first - 1] == term) {
+                    if (lane == 0) q[0] = (unsigned short)(first - 1u);
+                    qt = 1;
+                }
+                __syncwarp();
+                if (!inner) {
+                    if (lane < 3)
+                        W.edge[lane] = lane == 0 ? make_uint4(0u, 0u, 0u, 0u)
+                                                 : ral_txv_load16(R, lane == 1 ? lo_r & ~15u : hi_r & ~15u, lo_r, hi_r);
+                    __syncwarp();
+                }
+                // a granule inside the text is read where it lies, one at its ends or outside it from W.edge: the
+                // address is chosen, not the value, so the loads stay in flight until their step
+                auto granule = [&](ral_u32 at) {
+                    const uint4* p = reinterpret_cast<const uint4*>(R + at);
+                    if (!inner && (at < lo_r || at + 16u > hi_r))
+                        p = W.edge + (at + 16u <= lo_r || at >= hi_r ? 0 : at < lo_r ? 1 : 2);
+                    return *p;
+                };
+                uint4 u = granule(l32), v = granule(l32 + 16u);
+                ral_u32 off = 0;         // bytes staged
+                ral_u32 tm = 0;          // this lane's terminators of the last step that are not queued yet
+                bool left = false, end = false;
+                for (;;) {
+                    if (!left) {
+                        const bool in_range = off < RB && off < hi_r;
+                        bool step = in_range;
+                        ral_u32 e = 0u;
+                        if (!in_range) {
+                            // past the range (or the text): only the line that is still open matters
+                            const ral_u32 lead = qt ? (q[(qt - 1u) & RAL_QM] + 1u) & 0xffffu : RB;
+                            if (lead >= RB || lead >= hi_r) {
+                                end = true;
+                            } else if (off >= hi_r) {  // the text's last line has no terminator
+                                e = hi_r;
+                            } else if (off >= RB + RAL_RING) {
+                                // longer than the ring: its end is searched, its bytes are read from global memory
+                                last_end = hi;
+                                for (ral_i64 p = base + off; p < hi; p += 512) {
+                                    const ral_i64 at = p + 16 * lane;
+                                    const ral_u32 n = at < hi ? (ral_u32)(hi - at < 16 ? hi - at : 16) : 0u;
+                                    const ral_u32 m = n ? ral_txv_eq16(ral_txv_load16(A + at, 0u, 0u, n), T4) & ((1u << n) - 1u) : 0u;
+                                    const ral_u32 b = __ballot_sync(0xffffffffu, m != 0u);
+                                    if (b) {
+                                        const int l = __ffs(b) - 1;
+                                        last_end = p + 16 * l + __ffs(__shfl_sync(0xffffffffu, m, l)) - 1;
+                                        break;
+                                    }
+                                }
+                                e = 0xffffu;
+                            } else {
+                                step = true;
+                            }
+                        }
+                        if (step) {
+                            // this lane's 32 bytes into the ring, their delimiter bits, their terminators
+                            const ral_u32 rel = off + l32;
+                            *reinterpret_cast<uint4*>(tx + ((rel >> 2) & RAL_TXM)) = u;
+                            *reinterpret_cast<uint4*>(tx + ((rel >> 2) & RAL_TXM) + 4) = v;
+)RALK";
+    if (delims)
+        os << "                            W.db[(rel >> 5) & RAL_DBM] = ral_txv_eq16(u, D4) | ral_txv_eq16(v, D4) << 16;\n";
+    os << R"RALK(                            tm = ral_txv_eq16(u, T4) | ral_txv_eq16(v, T4) << 16;
+                            if (!inner) {  // positions outside [first, hi) end no line
+                                if (rel < first) tm &= first - rel >= 32u ? 0u : 0xffffffffu << (first - rel);
+                                if (rel + 32u > hi_r) tm &= rel >= hi_r ? 0u : (1u << (hi_r - rel)) - 1u;
+                            }
+                            u = granule(rel + 1024u);
+                            v = granule(rel + 1040u);
+                            if (!in_range) {
+                                const ral_u32 b = __ballot_sync(0xffffffffu, tm != 0u);
+                                if (b) {  // the first terminator past the range
+                                    const int l = __ffs(b) - 1;
+                                    e = off + 32u * l + __ffs(__shfl_sync(0xffffffffu, tm, l)) - 1u;
+                                }
+                                tm = 0u;
+                            }
+                            off += 1024u;
+                        }
+                        if (e) {
+                            if (lane == 0) q[qt & RAL_QM] = (unsigned short)e;
+                            qt += 1u;
+                            end = true;
+                        }
+                    }
+                    left = false;
+                    if (__any_sync(0xffffffffu, (tm & (tm - 1u)) != 0u)) {
+                        const ral_u32 c = __popc(tm);
+                        ral_u32 inc = c;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const ral_u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+                            if (lane >= o) inc += t;
+                        }
+                        // the lanes whose terminators fit now; the others' are queued after the next slices
+                        const bool fits = inc <= RAL_QM - 64u;
+                        if (fits)
+                            for (ral_u32 at = qt + inc - c; tm; tm &= tm - 1u)
+                                q[at++ & RAL_QM] = (unsigned short)(off - 1024u + l32 + __ffs(tm) - 1);
+                        qt += __reduce_max_sync(0xffffffffu, fits ? inc : 0u);
+                        left = __any_sync(0xffffffffu, tm != 0u);
+                    } else {
+                        const ral_u32 b = __ballot_sync(0xffffffffu, tm != 0u);
+                        if (tm) q[(qt + __popc(b & below)) & RAL_QM] = (unsigned short)(off - 1024u + l32 + __ffs(tm) - 1);
+                        qt += __popc(b);
+                        tm = 0u;
+                    }
+                    __syncwarp();
+                    // slices of 32 lines, one a lane; all that is queued at the end and where the next step would
+                    // overwrite the oldest line
+                    while (qt - qh > 1u) {
+                        const ral_u32 m = qt - qh - 1u < 32u ? qt - qh - 1u : 32u;
+                        if (m < 32u && !end && off + 1024u - ((q[qh & RAL_QM] + 1u) & 0xffffu) <= RAL_RING) break;
+                        const ral_u32 s = (q[(qh + lane) & RAL_QM] + 1u) & 0xffffu;
+                        const ral_u32 x = q[(qh + lane + 1u) & RAL_QM];
+                        bool keep = false;
+                        if ((ral_u32)lane < m && x != s) {
+                            const char* const ls = R + s;
+                            if (x != 0xffffu && off - s <= RAL_RING) {
+                                const ral_u32 z = ral_txv_byte<RAL_TXM>(tx, x - 1u) == '\r' ? x - 1u : x;
+                                keep = z != s;
+)RALK";
+    if (pred)
+        os << "                                if (keep) {\n                                    ral_u32 rf = 0u;\n"
+              "                                    keep = ral_keep(P, tx, " << (delims ? "W.db" : "(const ral_u32*)0") << ", s, z, ls, rf);\n"
+              "                                    if (pass == 0) refused += rf;\n                                }\n";
+    os << R"RALK(                            } else {
+                                ral_i64 n = x != 0xffffu ? (ral_i64)(x - s) : last_end - (base + s);
+                                if (ls[n - 1] == '\r') --n;
+                                keep = n > 0;
+)RALK";
+    if (pred)
+        os << "                                if (keep) {\n                                    const ral_u32 r = ral_keep_long(P, ls, n, "
+           << (delims ? "(char)(P.s[6] & 0xffu)" : "(char)0") << ");\n"
+              "                                    keep = (r & 1u) != 0u;\n"
+              "                                    if (pass == 0) refused += r >> 1;\n                                }\n";
+    os << R"RALK(                            }
+                        }
+                        const ral_u32 b = __ballot_sync(0xffffffffu, keep);
+                        const ral_u32 at = total + __popc(b & below);
+                        const ral_u32 n = x != 0xffffu ? x - s : 0xffffu;
+                        if (pass == 0) {
+                            if (keep && at < RAL_KL) W.kl[buf][at] = s | n << 16;
+                        } else if (keep && excl + at < cap) {
+                            list[excl + at] = (ral_u64)(base + s) | (ral_u64)n << 48;
+                        }
+                        total += __popc(b);
+                        qh += m;
+                    }
+                    __syncwarp();
+                    if (end && !left && qt - qh <= 1u) break;
+                }
+            }
+            if (pass) break;
+            ral_lookback_publish(status, range, total);
+            if (rangeA >= 0) write_list(rangeA, totalA, W.kl[buf ^ 1u]);
+            rangeA = -1;
+            if (total <= RAL_KL) {
+                rangeA = range;
+                totalA = total;
+                buf ^= 1u;
+                break;
+            }
+            excl = write_list(range, total, W.kl[buf]);
+        }
+    }
+    if (rangeA >= 0) write_list(rangeA, totalA, W.kl[buf ^ 1u]);
+    const ral_u32 rf = __reduce_add_sync(0xffffffffu, refused);
+    const ral_u32 ov = __reduce_add_sync(0xffffffffu, over);
+)RALK";
+    os << "    if (lane == 0 && rf) atomicAdd((unsigned long long*)(scratch + " << 3 + NP << "), (unsigned long long)rf);\n";
+    os << "    if (lane == 0 && ov) atomicAdd((unsigned long long*)(scratch + " << 4 + NP << "), (unsigned long long)ov);\n";
+    os << "}\n";
+    gk.source = os.str();
+    return gk;
+}
+
+// The second kernel: the projected fields of the listed lines, one line a lane, 32 consecutive kept
+// rows a warp and step.  The warp copies its lines' text to shared memory as it makes their delimiter
+// bits: their whole span where it is short (dense kept rows), else each line to a slot of its own,
+// eight lanes a line.  Stores are contiguous and each column's 32 validity bits come from one ballot.
+// Lines of more than 240 bytes are read from global memory byte by byte.
+GeneratedKernel generate_text_rows_kernel(const TextScanSpec& t, const Shape& s) {
+    GeneratedKernel gk;
+    gk.shape = s;
+    const TextScanParts parts = text_scan_parts(t);
+    gk.layout = parts.L;
+    const ParamLayout& L = gk.layout;
+    const int NP = (int)t.dtypes.size();
+    std::ostringstream key;
+    key << "textrows|" << parts.key << "|T" << s.threads << "B" << s.min_blocks;
+    char hex[32];
+    snprintf(hex, sizeof hex, "%016llx", (unsigned long long)fnv1a(key.str()));
+    gk.name = std::string("ral_textrows_") + hex;
+    gk.soft_fp = true;
+
+    std::ostringstream os;
+    os << ral_textscan_source << "\n";
+    os << "// generated: " << key.str() << "\n";
+    os << "#define RAL_THREADS " << s.threads << "\n#define RAL_WARPS (RAL_THREADS / 32)\n";
+    // the area: 16 bytes to spare, then 32 slots of 17 granules of 16 bytes (the odd count spreads
+    // the slots over the banks), 16 bytes to spare
+    os << "#define RAL_SLOT 272u\n#define RAL_AREA (32u + 32u * RAL_SLOT)\n#define RAL_SPAN 8192u\n";
+    os << "#define RAL_TXM 0xffffffffu\n#define RAL_DBM 0xffffffffu\n";
+    os << "struct RalParams { ral_u64 s[" << L.total << "]; };\n\n";
+    emit_text_finders(os, parts.f2);
+    std::string args, slow_vars, slow_call, slow_copy;
+    for (int q = 0; q < NP; q++) {
+        const bool isf = t.dtypes[q] == GDF_FLOAT32 || t.dtypes[q] == GDF_FLOAT64;
+        text_slow_vars(std::to_string(q), isf, slow_vars, slow_call, slow_copy);
+        args += std::string(", ") + (isf ? "double& x" : "ral_i64& x") + std::to_string(q) + ", ral_u32& w" + std::to_string(q);
+    }
+    os << "static __device__ __noinline__ void ral_line_slow(const char* ls, ral_i64 n, char delim, ral_u32& refused" << args
+       << ") {\n";
+    os << "    ral_i64 fs[" << parts.f2.size() << "], fe[" << parts.f2.size() << "];\n    ral_fields_slow(ls, n, delim, fs, fe);\n";
+    for (int q = 0; q < NP; q++)
+        emit_text_parse(os, "    ", t.dtypes[q], std::to_string(text_slot_of(parts.f2, t.file_cols[q])), "x" + std::to_string(q),
+                        "w" + std::to_string(q), false);
+    os << "}\n";
+    os << "\nextern \"C\" __global__ void __launch_bounds__(RAL_THREADS, " << std::max(1, s.min_blocks) << ") " << gk.name
+       << "(const __grid_constant__ RalParams P) {\n";
+    os << "    __shared__ __align__(16) ral_u32 s_tx[RAL_WARPS][RAL_AREA / 4u];\n";
+    os << "    __shared__ ral_u32 s_db[RAL_WARPS][RAL_AREA / 32u + 1u];\n";
+    emit_text_params(os, true);
+    os << "    const ral_u64 obase = (ral_u64)P.s[8];\n";
+    os << "    ral_u64* const scratch = (ral_u64*)P.s[" << L.scratch << "];\n";
     for (int q = 0; q < NP; q++) {
         os << "    " << element_ctype(t.dtypes[q]) << "* __restrict__ o" << q << " = (" << element_ctype(t.dtypes[q])
            << "*)P.s[" << L.out_data + q << "];\n";
         os << "    ral_u32* __restrict__ ov" << q << " = (ral_u32*)P.s[" << L.out_valid + q << "];\n";
     }
-    os << "    const int lane = threadIdx.x & 31;\n    const int warp = threadIdx.x >> 5;\n";
-    os << "    ral_u32* const s_kpw = s_kp[warp];\n    unsigned short* const s_lst = s_ls[warp];\n";
-    os << "    char* const s_txw = s_tx[warp];\n";
-    os << "    const ral_i64 CL = 32 * RAL_J;\n    const ral_i64 nchunks = (T + CL - 1) / CL;\n";
     os << "    ral_u32 vcnt[" << NP << "];\n    for (int q = 0; q < " << NP << "; ++q) vcnt[q] = 0u;\n";
-    os << "    ral_u32 refused = 0, over = 0;\n";
-    os << "    for (;;) {\n";
-    os << "        ral_u32 ticket = 0;\n";
-    os << "        if (lane == 0) ticket = atomicAdd((unsigned int*)scratch, 1u);\n";
-    os << "        const ral_i64 chunk = __shfl_sync(0xffffffffu, ticket, 0);\n";
-    os << "        if (chunk >= nchunks) break;\n";
-    os << "        const ral_i64 base = chunk * CL;\n";
-    os << "        ral_u32 total = 0;\n";
-    os << "        for (int j = 0; j < RAL_J; ++j) {\n";
-    os << "            const ral_i64 i0 = base + (ral_i64)j * 32;\n";
-    os << "            if (i0 >= T) {\n";
-    os << "                if (lane == j) s_kpw[j] = 0u;\n";
-    os << "                continue;\n";
-    os << "            }\n";
-    os << "            const ral_i64 i = i0 + lane;\n";
-    os << "            const char* ds = d;\n";
-    if (pred) {
-        // the slice's lines staged only when the condition has fields to parse
-        os << "            {\n";
-        os << "                const ral_i64 i1 = i0 + 31 < T ? i0 + 31 : T - 1;\n";
-        os << "                const ral_i64 S = i0 == 0 ? 0 : ends[i0 - 1] + 1;\n";
-        os << "                const ral_i64 E = i1 < nterm ? ends[i1] : nb;\n";
-        os << "                ds = ral_text_stage(d, nb, S, E, s_txw, lane);\n";
-        os << "            }\n";
-    }
-    os << "            bool keep = false;\n";
-    os << "            if (i < T && i >= skip) {\n";
-    os << "                ral_i64 s, e;\n";
-    os << "                ral_text_line(ds, ends, nterm, nb, i, s, e);\n";
-    os << "                keep = e > s;\n";
-    if (pred) {
-        os << "                if (keep) {\n";
-        if (!f1.empty()) {
-            os << "                    ral_i64 fs[" << f1.size() << "], fe[" << f1.size() << "];\n";
-            os << "                    ral_fields_pred(ds, s, e, delim, fs, fe);\n";
+    os << R"RALK(
+    ral_u32* const tx = s_tx[warp];
+    ral_u32* const db = s_db[warp];
+    unsigned short* const db16 = reinterpret_cast<unsigned short*>(db);
+    ral_u32 refused = 0;
+    auto text16 = [&](ral_i64 at) {  // 16 text bytes at a multiple of 16
+        const ral_u32 b0 = at < lo ? (ral_u32)(lo - at) : 0u;
+        const ral_u32 b1 = hi - at < 16 ? (ral_u32)(hi - at) : 16u;
+        return ral_txv_load16(A + at, 0u, b0, b1);
+    };
+    const ral_u64 kept = scratch[2] < cap ? scratch[2] : cap;
+    const ral_u64 step = (ral_u64)gridDim.x * RAL_THREADS;
+    for (ral_u64 k0 = ((ral_u64)blockIdx.x * RAL_WARPS + warp) * 32u; k0 < kept; k0 += step) {
+        const bool act = k0 + lane < kept;
+        const ral_u64 ent = act ? list[k0 + lane] : 0ull;
+        const ral_i64 g = (ral_i64)(ent & 0xffffffffffffull);
+        ral_i64 n = (ral_i64)(ent >> 48);
+        const int m = (int)(kept - k0 < 32u ? kept - k0 : 32u);
+        const bool lng = n == 65535;
+        if (act && lng) {
+            n = 0;
+            while (g + n < hi && A[g + n] != term) ++n;
         }
-        os << "                    ral_u32 fv[" << std::max<size_t>(1, t.predicate_cols.size()) << "];\n";
-        for (size_t c = 0; c < t.predicate_cols.size(); c++) {
-            const int q = t.predicate_cols[c];
-            if (!(pred_ref[c] || pred_raw[c])) {
-                os << "                    fv[" << c << "] = 0xffffffffu;\n";
-                continue;
+        const ral_i64 a0 = __shfl_sync(0xffffffffu, g, 0) & ~15ll;
+        const ral_i64 zl = __shfl_sync(0xffffffffu, g + n, m - 1);
+        const bool any_long = __any_sync(0xffffffffu, act && lng);
+        ral_u32 s = 16u;
+        bool in = true;
+        __syncwarp();
+        if (!any_long && zl - a0 <= (ral_i64)RAL_SPAN) {
+            for (ral_u32 o = 16u * lane; (ral_i64)o < zl - a0; o += 512u) {
+                const uint4 v = text16(a0 + o);
+                *reinterpret_cast<uint4*>(tx + ((16u + o) >> 2)) = v;
+                db16[(16u + o) >> 4] = (unsigned short)ral_txv_eq16(v, D4);
             }
-            parse("                    ", t.dtypes[q], std::to_string(slot_of(f1, t.file_cols[q])), "x" + std::to_string(c),
-                  "w" + std::to_string(c), "true");
-            os << "                    fv[" << c << "] = w" << c << ";\n";
+            if (act) s = 16u + (ral_u32)(g - a0);
+        } else {
+            const ral_i64 ng = ((g & 15) + n + 15) >> 4;
+            in = ng <= 16;
+            const int gr = act && in ? (int)ng : 0;
+            const int most = __reduce_max_sync(0xffffffffu, gr);
+            for (int h = 0; h < most; h += 8)
+                for (int it = 0; it < 8; ++it) {
+                    const int l = it * 4 + (lane >> 3), c = h + (lane & 7);
+                    const ral_i64 gl = __shfl_sync(0xffffffffu, g, l);
+                    if (c < __shfl_sync(0xffffffffu, gr, l)) {
+                        const uint4 v = text16((gl & ~15ll) + 16 * c);
+                        const ral_u32 o = 16u + l * RAL_SLOT + 16u * c;
+                        *reinterpret_cast<uint4*>(tx + (o >> 2)) = v;
+                        db16[o >> 4] = (unsigned short)ral_txv_eq16(v, D4);
+                    }
+                }
+            s = 16u + lane * RAL_SLOT + (ral_u32)(g & 15);
         }
-        os << "                    " << kind_ctype(pred_kind[0]) << " y0;\n";
-        os << "                    ral_pred_row(P";
-        for (size_t c = 0; c < t.predicate_cols.size(); c++)
-            if (pred_ref[c]) os << ", x" << c;
-        for (size_t c = 0; c < t.predicate_cols.size(); c++)
-            if (pred_raw[c]) os << ", w" << c << " & 1u";
-        os << ", y0);\n";
-        os << "                    keep = (ral_pred_vrow(fv) & 1u) != 0u && " << narrow("y0", pred_kind[0], GDF_INT8)
-           << " != 0;\n";
-        os << "                }\n";
-    }
-    os << "            }\n";
-    os << "            const ral_u32 w = __ballot_sync(0xffffffffu, keep);\n";
-    os << "            if (lane == j) s_kpw[j] = w;\n";
-    os << "            total += __popc(w);\n";
-    os << "        }\n";
-    os << "        __syncwarp();\n";
-    os << "        const ral_u64 excl = ral_lookback(status, chunk, total, scratch + 1);\n";
-    os << "        if (chunk == nchunks - 1 && lane == 0) scratch[2] = excl + total;\n";
-    os << "        if (total == 0u) continue;\n";
-    os << "        {\n";
-    os << "            const ral_u32 kw = lane < RAL_J ? s_kpw[lane] : 0u;\n";
-    os << "            const ral_u32 c = __popc(kw);\n";
-    os << "            ral_u32 inc = c;\n";
-    os << "            for (int off = 1; off < 32; off <<= 1) {\n";
-    os << "                const ral_u32 u = __shfl_up_sync(0xffffffffu, inc, off);\n";
-    os << "                if (lane >= off) inc += u;\n            }\n";
-    os << "            ral_u32 q = inc - c;\n";
-    os << "            for (ral_u32 m = kw; m; m &= m - 1u) s_lst[q++] = (unsigned short)(lane * 32 + __ffs(m) - 1);\n";
-    os << "        }\n";
-    os << "        __syncwarp();\n";
-    os << "        for (ral_u32 k0 = 0; k0 < total; k0 += 32) {\n";
-    os << "            const ral_u32 kA = k0 + lane;\n";
-    os << "            const bool act = kA < total;\n";
-    os << "            const ral_i64 i = base + s_lst[act ? kA : k0];\n";
-    os << "            const char* ds = d;\n";
-    os << "            {\n";
-    os << "                const ral_i64 i0 = base + s_lst[k0];\n";
-    os << "                const ral_i64 i1 = base + s_lst[k0 + 31u < total ? k0 + 31u : total - 1u];\n";
-    os << "                const ral_i64 S = i0 == 0 ? 0 : ends[i0 - 1] + 1;\n";
-    os << "                const ral_i64 E = i1 < nterm ? ends[i1] : nb;\n";
-    os << "                ds = ral_text_stage(d, nb, S, E, s_txw, lane);\n";
-    os << "            }\n";
-    os << "            ral_i64 s, e;\n";
-    os << "            ral_text_line(ds, ends, nterm, nb, i, s, e);\n";
-    os << "            ral_i64 fs[" << f2.size() << "], fe[" << f2.size() << "];\n";
-    os << "            ral_fields_all(ds, s, e, delim, fs, fe);\n";
-    os << "            const ral_u64 pos0 = excl + kA;\n";
-    os << "            const bool put = act && pos0 < cap;\n";
-    os << "            if (act && !put) ++over;\n";
-    os << "            const ral_u64 pos = pos0 + obase;\n";
-    os << "            const ral_u64 b = excl + k0 + obase;\n";
+        __syncwarp();
+        const char* const ls = A + g;
+)RALK";
     for (int q = 0; q < NP; q++) {
-        os << "            {\n";
-        parse("                ", t.dtypes[q], std::to_string(slot_of(f2, t.file_cols[q])), "v", "vw", "act");
-        os << "                if (put) o" << q << "[pos] = (" << element_ctype(t.dtypes[q]) << ")v;\n";
-        os << "                const ral_u32 bal = __ballot_sync(0xffffffffu, put && vw != 0u);\n";
-        os << "                if (lane == 0 && bal) {\n";
-        os << "                    vcnt[" << q << "] += __popc(bal);\n";
-        os << "                    const ral_u64 X = (ral_u64)bal << (b & 31u);\n";
-        os << "                    atomicOr(ov" << q << " + (b >> 5), (ral_u32)X);\n";
-        os << "                    if ((ral_u32)(X >> 32)) atomicOr(ov" << q << " + (b >> 5) + 1, (ral_u32)(X >> 32));\n";
-        os << "                }\n";
-        os << "            }\n";
+        const bool isf = t.dtypes[q] == GDF_FLOAT32 || t.dtypes[q] == GDF_FLOAT64;
+        os << "        " << (isf ? "double x" : "ral_i64 x") << q << " = 0;\n        ral_u32 w" << q << " = 0u;\n";
     }
-    os << "        }\n";
-    os << "        __syncwarp();\n";
+    os << "        if (act) {\n";
+    os << "            if ((in ? ral_txv_byte<RAL_TXM>(tx, s + (ral_u32)n - 1u) : (ral_u32)(unsigned char)ls[n - 1]) == '\\r') --n;\n";
+    os << "            if (in) {\n";
+    os << "                ral_u32 fs[" << parts.f2.size() << "], fe[" << parts.f2.size()
+       << "];\n                ral_fields(db, s, s + (ral_u32)n, fs, fe);\n";
+    for (int q = 0; q < NP; q++)
+        emit_text_parse(os, "                ", t.dtypes[q], std::to_string(text_slot_of(parts.f2, t.file_cols[q])),
+                        "x" + std::to_string(q), "w" + std::to_string(q), true);
+    os << "            } else {\n                ral_u32 rf = 0u;\n                " << slow_vars
+       << "\n                ral_line_slow(ls, n, (char)(P.s[6] & 0xffu), rf" << slow_call << ");\n                " << slow_copy
+       << "refused += rf;\n            }\n        }\n";
+    os << "        const ral_u64 b = k0 + obase;\n";
+    for (int q = 0; q < NP; q++) {
+        os << "        {\n";
+        os << "            if (act) o" << q << "[b + lane] = (" << element_ctype(t.dtypes[q]) << ")x" << q << ";\n";
+        os << "            const ral_u32 bal = __ballot_sync(0xffffffffu, w" << q << " != 0u);\n";
+        os << "            if (lane == 0 && bal) {\n";
+        os << "                vcnt[" << q << "] += __popc(bal);\n";
+        os << "                const ral_u64 X = (ral_u64)bal << (b & 31u);\n";
+        os << "                atomicOr(ov" << q << " + (b >> 5), (ral_u32)X);\n";
+        os << "                if ((ral_u32)(X >> 32)) atomicOr(ov" << q << " + (b >> 5) + 1, (ral_u32)(X >> 32));\n";
+        os << "            }\n        }\n";
+    }
     os << "    }\n";
-    // counts: one atomic per warp and counter
     os << "    for (int q = 0; q < " << NP << "; ++q) {\n";
     os << "        const ral_u32 v = __reduce_add_sync(0xffffffffu, vcnt[q]);\n";
     os << "        if (lane == 0 && v) atomicAdd((unsigned long long*)(scratch + 3 + q), (unsigned long long)v);\n";
     os << "    }\n";
     os << "    const ral_u32 rf = __reduce_add_sync(0xffffffffu, refused);\n";
-    os << "    const ral_u32 ov = __reduce_add_sync(0xffffffffu, over);\n";
     os << "    if (lane == 0 && rf) atomicAdd((unsigned long long*)(scratch + " << 3 + NP << "), (unsigned long long)rf);\n";
-    os << "    if (lane == 0 && ov) atomicAdd((unsigned long long*)(scratch + " << 4 + NP << "), (unsigned long long)ov);\n";
     os << "}\n";
     gk.source = os.str();
     return gk;

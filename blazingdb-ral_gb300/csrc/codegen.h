@@ -225,17 +225,23 @@ struct TextScanSpec {
     const Program* predicate = nullptr;  // the LogicalFilter's program, or none (the scan alone)
     std::vector<int> predicate_cols;     // scanned-frame column of each predicate input
 };
-// Scratch of a text scan launch: ticket, look-back error, kept rows, one valid count per output,
-// refused fields, rows past the outputs' capacity; then one status word per chunk.
-inline int64_t text_scan_header(int n_outputs) { return 5 + n_outputs; }
-// Parameter slots before the outputs: lines, text, bytes, terminator positions, terminators,
-// rows skipped, delimiter, output capacity, output row base (0 .. 31: kept row j is written at
-// row base + j of the output pointers and masks, which a piece of a longer scan appends into a
-// mask word the rows before it have started).
+// Scratch of a text scan: ticket, look-back error, kept rows, one valid count per output, refused
+// fields, rows past the outputs' capacity, bytes before the first line scanned; then one status word
+// per range.
+inline int64_t text_scan_header(int n_outputs) { return 6 + n_outputs; }
+// Parameter slots before the outputs: ranges, the text's address rounded down to 16 bytes, the
+// text's end and start relative to it, the kept-line list, bytes per range, delimiter and terminator
+// (delimiter | terminator << 8), list capacity, output row base (0 .. 31: kept row j is written at
+// row base + j of the output pointers and masks, which a piece of a longer scan appends into a mask
+// word the rows before it have started).
 constexpr int kTextScanFixedSlots = 9;
-// Lines per look-back chunk of a text scan kernel: J mask words of 32 lines.
-inline int64_t text_scan_chunk_lines(const Shape& s) { return (int64_t)32 * s.J; }
+// The most text bytes a warp of the scan takes at a time (a multiple of 1024; positions in a range, which
+// reach a ring's length and a step past its end, are 16-bit), and the kept lines of a range that wait in
+// shared memory (a range with more is read twice).
+constexpr int64_t kTextScanRangeBytes = 49152;
+constexpr int64_t kTextScanKeptLines = 512;
 
 GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s);
+GeneratedKernel generate_text_rows_kernel(const TextScanSpec& t, const Shape& s);
 
 }  // namespace ral

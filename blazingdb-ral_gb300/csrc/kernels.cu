@@ -479,6 +479,51 @@ __global__ void __launch_bounds__(256) text_term_positions_kernel(const char* __
     }
 }
 
+// One block: the tile holding the k-th terminator from the tiles' offsets (or the first one), then
+// steps of 4 KiB until it is reached.
+__global__ void __launch_bounds__(256) text_skip_kernel(const char* __restrict__ data, int64_t n, char term, int64_t k,
+                                                        const unsigned long long* __restrict__ offsets, int64_t tiles,
+                                                        unsigned long long* __restrict__ out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ ral_u32 s_w[2][8];
+    int64_t at0 = 0, seen = 0;
+    if (offsets) {
+        int64_t a = 0, b = tiles;  // the last tile with fewer than k terminators before it
+        while (b - a > 1) {
+            const int64_t m = (a + b) / 2;
+            if ((int64_t)offsets[m] < k) a = m;
+            else b = m;
+        }
+        at0 = a * kTextTileBytes;
+        seen = (int64_t)offsets[a];
+    }
+    for (int i = 0; at0 < n; ++i, at0 += kTextStepBytes) {
+        const int64_t at = at0 + 16 * (int64_t)threadIdx.x;
+        ral_u32 bits = ral_text_term_bits(data, n, at, term);
+        const ral_u32 c = __popc(bits);
+        ral_u32 inc = c;
+        for (int off = 1; off < 32; off <<= 1) {
+            const ral_u32 t = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += t;
+        }
+        if (lane == 31) s_w[i & 1][warp] = inc;
+        __syncthreads();
+        int64_t before = seen + inc - c, total = seen;
+        for (int w = 0; w < 8; ++w) {
+            const ral_u32 x = s_w[i & 1][w];
+            if (w < warp) before += x;
+            total += x;
+        }
+        if (before < k && before + c >= k) {
+            for (int64_t j = before + 1; j < k; ++j) bits &= bits - 1u;
+            *out = (unsigned long long)(at + __ffs(bits));
+        }
+        if (total >= k) return;  // block-uniform
+        seen = total;
+    }
+    if (threadIdx.x == 0) *out = (unsigned long long)n;
+}
+
 __global__ void __launch_bounds__(256) text_present_count_kernel(const char* __restrict__ data, int64_t n,
                                                                  const long long* __restrict__ ends, int64_t nterm,
                                                                  int64_t lines, int64_t skip,
@@ -516,6 +561,13 @@ cudaError_t launch_text_term_counts(const char* data, int64_t n, char term, uint
 cudaError_t launch_exclusive_scan_u32(const uint32_t* counts, int64_t tiles, unsigned long long* offsets,
                                       cudaStream_t st) {
     exclusive_scan_u32_kernel<<<1, 1024, 0, st>>>(counts, tiles, offsets);
+    note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_text_skip(const char* data, int64_t n, char term, int64_t k, const unsigned long long* offsets,
+                             unsigned long long* out, cudaStream_t st) {
+    text_skip_kernel<<<1, 256, 0, st>>>(data, n, term, k, offsets, text_tiles(n), out);
     note_launch();
     return cudaGetLastError();
 }

@@ -59,6 +59,10 @@ cudaError_t launch_text_term_counts(const char* data, int64_t n, char term, uint
 // offsets[t] = counts[0] + .. + counts[t-1] for t <= tiles (offsets[tiles] = the total), one block.
 cudaError_t launch_exclusive_scan_u32(const uint32_t* counts, int64_t tiles, unsigned long long* offsets,
                                       cudaStream_t st);
+// *out = the byte after the k-th (k >= 1) line terminator of data[0, n), n when there are fewer.
+// offsets: launch_exclusive_scan_u32's over data's tiles, or null (data is read from its start).
+cudaError_t launch_text_skip(const char* data, int64_t n, char term, int64_t k, const unsigned long long* offsets,
+                             unsigned long long* out, cudaStream_t st);
 // ends[k] = position of the k-th line terminator of data[0, n), in order.
 cudaError_t launch_text_term_positions(const char* data, int64_t n, char term, const unsigned long long* offsets,
                                        long long* ends, cudaStream_t st);

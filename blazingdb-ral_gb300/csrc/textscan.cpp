@@ -4,11 +4,10 @@
 // `projects=[...]` list picks the file columns) through csv_parser::parse
 // (src/io/data_parser/CSVParser.cpp:176-233, cudf's CSV reader), and a LogicalFilter above the
 // scan then evaluates its condition over the scanned frame and compacts it
-// (CalciteInterpreter.cpp:509-573).  Here the text stays in device memory and the two run as one:
-// a line index (three small kernels: terminators per tile, a scan, their positions), then one
-// generated kernel that parses the predicate's fields of every line, evaluates the predicate,
-// finds each chunk's output offset by look-back and parses and stores the projected fields of the
-// kept lines only.  Field rules: csrc/textscan.cuh.
+// (CalciteInterpreter.cpp:509-573).  Here the text stays in device memory and the two run as two
+// generated kernels: one finds every line, parses the predicate's fields, evaluates the predicate and
+// lists the kept lines in order (look-back over the text's ranges), the other parses and stores the
+// projected fields of the listed lines.  Field rules: csrc/textscan.cuh.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -91,22 +90,41 @@ int build_line_index(const char* data, int64_t n, char term, cudaStream_t st, Li
                       "line terminator positions");
 }
 
-// A compiled scan kernel with its predicate program (the program's scalars fill the launch).
+// Enqueues the search for the line after the first `lines` of data[0, n): its offset (n when there is
+// none) goes to *out, device memory.  A few lines (a header) are passed over by one block from the
+// front; more lines are looked up in the tiles' terminator counts.
+int skip_lines(const char* data, int64_t n, char term, int64_t lines, unsigned long long* out, cudaStream_t st) {
+    constexpr int64_t kFew = 16;
+    if (lines <= kFew)
+        return check_cuda(launch_text_skip(data, n, term, lines, nullptr, out, st), "skipped lines");
+    const int64_t tiles = text_tiles(n);
+    StreamBuffer counts(st), offsets(st);
+    if (int e = counts.alloc((size_t)tiles * 4)) return e;
+    if (int e = offsets.alloc((size_t)(tiles + 1) * 8)) return e;
+    if (int e = check_cuda(launch_text_term_counts(data, n, term, (uint32_t*)counts.p, st), "line terminators")) return e;
+    if (int e = check_cuda(launch_exclusive_scan_u32((const uint32_t*)counts.p, tiles, (unsigned long long*)offsets.p, st),
+                           "line terminator scan"))
+        return e;
+    return check_cuda(launch_text_skip(data, n, term, lines, (const unsigned long long*)offsets.p, out, st), "skipped lines");
+}
+
+// A scan's two compiled kernels with the predicate program (whose scalars fill the launches).
 struct PreparedScan {
     Program pred;
     bool have_pred = false;
     TextScanSpec spec;
-    GeneratedKernel gk;
+    GeneratedKernel gk, gk_rows;  // the condition over every line; the kept lines' fields
     const CompiledKernel* k = nullptr;
+    const CompiledKernel* k_rows = nullptr;
 };
 std::mutex g_scan_mu;
 std::map<std::string, std::unique_ptr<PreparedScan>> g_scans;
 
 Shape text_scan_shape() {
+    // four warps a block, whose rings and bitmaps take 43 KB of shared memory: five blocks an SM
     Shape s;
-    s.J = 8;  // 256 lines per look-back chunk
-    s.threads = 256;
-    s.min_blocks = 4;
+    s.threads = 128;
+    s.min_blocks = 5;
     apply_shape_tune(s, std::getenv("RAL_SCAN_TUNE") ? std::getenv("RAL_SCAN_TUNE") : "");
     return s;
 }
@@ -151,6 +169,7 @@ int build_scan(const std::vector<gdf_dtype>& dtypes, const std::vector<int>& fil
         ps->spec.predicate_cols = ep.input_columns;
     }
     ps->gk = generate_text_scan_kernel(ps->spec, text_scan_shape());
+    ps->gk_rows = generate_text_rows_kernel(ps->spec, text_scan_shape());
     return kSuccess;
 }
 
@@ -159,7 +178,7 @@ int prepare_scan(const std::vector<gdf_dtype>& dtypes, const std::vector<int>& f
     const Shape sh = text_scan_shape();
     std::string key = std::string(filter_q ? filter_q : "") + "|";
     for (size_t q = 0; q < dtypes.size(); q++) key += std::to_string((int)dtypes[q]) + "@" + std::to_string(file_cols[q]) + ",";
-    key += "|J" + std::to_string(sh.J) + "T" + std::to_string(sh.threads) + "B" + std::to_string(sh.min_blocks);
+    key += "|T" + std::to_string(sh.threads) + "B" + std::to_string(sh.min_blocks);
     {
         std::lock_guard<std::mutex> lock(g_scan_mu);
         auto it = g_scans.find(key);
@@ -172,7 +191,8 @@ int prepare_scan(const std::vector<gdf_dtype>& dtypes, const std::vector<int>& f
     if (int e = build_scan(dtypes, file_cols, filter_q, *ps)) return e;
     std::string err;
     ps->k = jit_get(ps->gk, err);
-    if (!ps->k) return set_error(kJitError, err);
+    if (ps->k) ps->k_rows = jit_get(ps->gk_rows, err);
+    if (!ps->k || !ps->k_rows) return set_error(kJitError, err);
     std::lock_guard<std::mutex> lock(g_scan_mu);
     auto res = g_scans.emplace(key, std::move(ps));
     *out = res.first->second.get();
@@ -227,13 +247,16 @@ int text_scan_source(const int32_t* file_dtypes, int32_t n_file, const int32_t* 
     if (int e = scan_columns(file_dtypes, n_file, projections, n_proj, dtypes, file_cols)) return e;
     PreparedScan ps;
     if (int e = build_scan(dtypes, file_cols, filter_q, ps)) return e;
-    source = std::string(jit_prelude()) + "\n" + ps.gk.source;
+    source = std::string(jit_prelude()) + "\n" + ps.gk.source + "\n" + ps.gk_rows.source;
     if (compile) {
-        std::string err;
-        size_t bytes = 0;
-        if (!jit_compile_only(ps.gk, &bytes, &log, err)) {
-            log = err;
-            return set_error(kJitError, err);
+        for (const GeneratedKernel* gk : {&ps.gk, &ps.gk_rows}) {
+            std::string err, one;
+            size_t bytes = 0;
+            if (!jit_compile_only(*gk, &bytes, &one, err)) {
+                log = err;
+                return set_error(kJitError, err);
+            }
+            log += one;
         }
     }
     return kSuccess;
@@ -255,33 +278,51 @@ int check_outs(const std::vector<gdf_dtype>& dtypes, gdf_column* const* outs, in
     return kSuccess;
 }
 
-// One scan launch over data[0, n) (device memory): its kept rows go to rows row0 .. of the
-// outputs (whose masks are zeroed), at most cap of them; adds the rows kept and each output's
-// valid rows to kept / valid.  Synchronous on st.
-int scan_piece(const PreparedScan& ps, const char* data, int64_t n, char delim, char term, int32_t skip_rows,
-               gdf_column* const* outs, int NP, int64_t row0, int64_t cap, cudaStream_t st, int64_t& kept,
-               std::vector<int64_t>& valid) {
-    LineIndex li(st);
-    if (int e = build_line_index(data, n, term, st, li)) return e;
-    const GeneratedKernel& gk = ps.gk;
-    const ParamLayout& L = gk.layout;
-    const int64_t chunks = (li.lines + text_scan_chunk_lines(gk.shape) - 1) / text_scan_chunk_lines(gk.shape);
-    if (chunks == 0) return kSuccess;
+// Text bytes per range of n bytes of which at most `cap` lines are kept.  A range costs a look-back and
+// a last slice that is partly filled (20M lines of 62 bytes took 1009 / 905 / 865 us at 8 / 16 / 24 KiB), so
+// as many as the positions allow; less where the kept lines may be so short that more of them than wait
+// in shared memory come from one range, and for small texts, so that every warp the device holds gets one.
+int64_t range_bytes(int64_t n, int64_t cap) {
+    const int64_t warps = (int64_t)device_sms() * 20;
+    const int64_t spread = (n / warps + 1023) / 1024 * 1024;
+    const int64_t kept = (int64_t)((double)n / std::max<int64_t>(cap, 1) * (kTextScanKeptLines * 7 / 8)) / 1024 * 1024;
+    return std::max<int64_t>(1024, std::min({spread, kept, kTextScanRangeBytes}));
+}
+
+// The lines of data[0, n) (device memory) that start at or after byte `from` (where a line starts),
+// less the first skip_rows of them: the kept rows go to rows row0 .. of the outputs (whose masks are
+// zeroed), at most cap of them; adds the rows kept and each output's valid rows to kept / valid.
+// Synchronous on st.
+int scan_piece(const PreparedScan& ps, const char* data, int64_t n, char delim, char term, int64_t from,
+               int32_t skip_rows, gdf_column* const* outs, int NP, int64_t row0, int64_t cap, cudaStream_t st,
+               int64_t& kept, std::vector<int64_t>& valid) {
+    if (n <= from) return kSuccess;
+    const ParamLayout& L = ps.gk.layout;
+    const int64_t head = (int64_t)((uintptr_t)data & 15);
+    const int64_t rb = range_bytes(n - from, cap);
+    const int64_t ranges = (head + n + rb - 1) / rb;
     const int64_t header = text_scan_header(NP);
-    StreamBuffer scratch(st);
-    if (int e = scratch.alloc((size_t)(header + chunks) * 8)) return e;
-    cudaMemsetAsync(scratch.p, 0, (size_t)(header + chunks) * 8, st);
+    cap = std::max<int64_t>(cap, 0);
+    // a kept line has at least one byte and, but for the last, a terminator
+    const int64_t listed = std::min(cap, (n - from + 1) / 2);
+    StreamBuffer scratch(st), list(st);
+    if (int e = scratch.alloc((size_t)(header + ranges) * 8)) return e;
+    if (int e = list.alloc((size_t)listed * 8)) return e;
+    cudaMemsetAsync(scratch.p, 0, (size_t)(header + ranges) * 8, st);
+    if (skip_rows > 0)
+        if (int e = skip_lines(data + from, n - from, term, skip_rows, (unsigned long long*)scratch.p + header - 1, st))
+            return e;
     // the outputs seen from the word holding row0: row (row0 & 31) + j is kept row j
     const int64_t obase = row0 & 31;
     std::vector<uint64_t> slots(L.total, 0);
-    slots[0] = (uint64_t)li.lines;
-    slots[1] = (uint64_t)(uintptr_t)data;
-    slots[2] = (uint64_t)n;
-    slots[3] = (uint64_t)(uintptr_t)li.ends.p;
-    slots[4] = (uint64_t)li.nterm;
-    slots[5] = (uint64_t)skip_rows;
-    slots[6] = (uint64_t)(unsigned char)delim;
-    slots[7] = (uint64_t)std::max<int64_t>(cap, 0);
+    slots[0] = (uint64_t)ranges;
+    slots[1] = (uint64_t)((uintptr_t)data & ~(uintptr_t)15);
+    slots[2] = (uint64_t)(head + n);
+    slots[3] = (uint64_t)(head + from);
+    slots[4] = (uint64_t)(uintptr_t)list.p;
+    slots[5] = (uint64_t)rb;
+    slots[6] = (uint64_t)(unsigned char)delim | (uint64_t)(unsigned char)term << 8;
+    slots[7] = (uint64_t)listed;  // cap, or more lines than the text can hold
     slots[8] = (uint64_t)obase;
     for (int q = 0; q < NP; q++) {
         const int64_t w = gdf_dtype_size(outs[q]->dtype);
@@ -294,11 +335,17 @@ int scan_piece(const PreparedScan& ps, const char* data, int64_t n, char delim, 
     // behind the host-to-device copies of a streamed scan
     thread_local unsigned long long* h = nullptr;
     if (!h && check_cuda(cudaMallocHost((void**)&h, 8 * 72), "cudaMallocHost")) return kCudaError;
-    const int grid = launch_blocks(*ps.k, gk.shape.threads, text_scan_chunk_lines(gk.shape) * (gk.shape.threads / 32),
-                                   li.lines);
     void* args[] = {slots.data()};
-    if (int e = check_cuda(cudaLaunchKernel((const void*)ps.k->kernel, dim3(grid), dim3(gk.shape.threads), args, 0, st),
+    const int threads = ps.gk.shape.threads;
+    const int grid = launch_blocks(*ps.k, threads, threads / 32, ranges);
+    if (int e = check_cuda(cudaLaunchKernel((const void*)ps.k->kernel, dim3(grid), dim3(threads), args, 0, st),
                            "launch of the text scan kernel"))
+        return e;
+    note_launch();
+    const int threads2 = ps.gk_rows.shape.threads;
+    const int grid2 = launch_blocks(*ps.k_rows, threads2, threads2, listed);
+    if (int e = check_cuda(cudaLaunchKernel((const void*)ps.k_rows->kernel, dim3(grid2), dim3(threads2), args, 0, st),
+                           "launch of the text rows kernel"))
         return e;
     note_launch();
     if (int e = check_cuda(cudaMemcpyAsync(h, scratch.p, (size_t)header * 8, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync"))
@@ -351,7 +398,7 @@ int text_scan_filter(const char* data, int64_t n, char delim, char term, int32_t
         if (cap > 0) cudaMemsetAsync(outs[q]->valid, 0, (size_t)((cap + 31) / 32) * 4, st);
     int64_t kept = 0;
     std::vector<int64_t> valid(NP, 0);
-    if (int e = scan_piece(*ps, data, n, delim, term, skip_rows, outs, NP, 0, cap, st, kept, valid)) return e;
+    if (int e = scan_piece(*ps, data, n, delim, term, 0, skip_rows, outs, NP, 0, cap, st, kept, valid)) return e;
     set_outputs(outs, NP, kept, valid, n_out);
     return kSuccess;
 }
@@ -377,8 +424,7 @@ int text_scan_filter_host(const char* text, int64_t n, char delim, char term, in
     }
     // pieces of whole lines: each ends just after a terminator (the last at the end of the text).
     // A piece is copied from the 256-byte boundary at or before its first line (copies from
-    // unaligned host addresses run slower, and the kernels read aligned text 16 bytes at a time);
-    // the lines before its first one there all end inside it and are skipped by the scan.
+    // unaligned host addresses run slower); the scan starts `skip` bytes in, at its first line.
     const int64_t P = piece_bytes();
     struct Piece {
         int64_t from, to, skip;
@@ -392,9 +438,7 @@ int text_scan_filter_host(const char* text, int64_t n, char delim, char term, in
             e0 = t ? (int64_t)((const char*)t - text) + 1 : n;
         }
         const int64_t a = s0 & ~(int64_t)255;
-        int64_t skip = 0;
-        for (int64_t p = a; p < s0; p++) skip += text[p] == term;
-        pieces.push_back({a, e0, skip});
+        pieces.push_back({a, e0, s0 - a});
         biggest = std::max(biggest, e0 - a);
         s0 = e0;
     }
@@ -439,7 +483,7 @@ int text_scan_filter_host(const char* text, int64_t n, char delim, char term, in
         if (int e = lane_event(*lane, k, &ev)) return e;
         if (int e = check_cuda(cudaStreamWaitEvent(st, ev, 0), "cudaStreamWaitEvent")) return e;
         if (int e = scan_piece(*ps, (const char*)bufs[k % NB]->p, pieces[k].to - pieces[k].from, delim, term,
-                               (int32_t)pieces[k].skip, outs, NP, kept, cap - kept, st, kept, valid))
+                               pieces[k].skip, 0, outs, NP, kept, cap - kept, st, kept, valid))
             return e;
     }
     set_outputs(outs, NP, kept, valid, n_out);
