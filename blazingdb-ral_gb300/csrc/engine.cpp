@@ -110,6 +110,7 @@ namespace {
 struct DeviceInfo {
     int sms = 0;             // 0: not read yet
     bool pool_kept = false;  // keep_pool_memory ran
+    cudaMemPool_t scratch = nullptr;
 };
 std::mutex g_dev_mu;
 std::unordered_map<int, DeviceInfo> g_devs;
@@ -140,6 +141,26 @@ void keep_pool_memory() {
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
     d.pool_kept = true;
+}
+
+int scratch_pool(cudaMemPool_t* out) {
+    int dev = 0;
+    if (int e = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return e;
+    std::lock_guard<std::mutex> lock(g_dev_mu);
+    DeviceInfo& d = g_devs[dev];
+    if (!d.scratch) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (int e = check_cuda(cudaMemPoolCreate(&pool, &props), "cudaMemPoolCreate")) return e;
+        uint64_t kept = kScratchPoolKept;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+        d.scratch = pool;
+    }
+    *out = d.scratch;
+    return kSuccess;
 }
 
 int copy_lane(CopyLane*& out) {

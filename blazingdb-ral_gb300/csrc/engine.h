@@ -90,6 +90,11 @@ int blocks_per_sm(const CompiledKernel& k, int threads);
 // server are reused rather than mapped again (set once per device for the process).
 void keep_pool_memory();
 
+// The pool of the current device for large per-call scratch (made once, shared by all threads): of what
+// calls have freed it keeps at most kScratchPoolKept bytes at a synchronisation.
+constexpr uint64_t kScratchPoolKept = (uint64_t)8 << 30;
+int scratch_pool(cudaMemPool_t* out);
+
 // The copy stream of the calling thread on the current device, with its events (made once, kept
 // for the thread's life): host-to-device copies issued on it overlap kernels on the caller's stream.
 struct CopyLane {

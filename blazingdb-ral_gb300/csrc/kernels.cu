@@ -109,7 +109,7 @@ cudaError_t gather_by_index(const void* in, const uint32_t* in_valid, int64_t n_
 // row-major order loads them normally).
 constexpr int kGatherRowsPerLane = 4;
 constexpr int kGatherSamples = 64;          // index samples of 32 consecutive rows
-constexpr long long kGatherClusterSpan = 1 << 16;  // a sample spanning fewer input rows is clustered
+constexpr ral_u32 kGatherClusterSpan = 1u << 16;  // a sample spanning fewer input rows is clustered
 
 template <typename I>
 __device__ __forceinline__ ral_i64 ral_load_index(const void* idx, ral_i64 i) {
@@ -181,20 +181,24 @@ __device__ __forceinline__ void ral_step_indices(const GatherColumnsParams& P, r
     }
 }
 
-// Clustered samples among the 32 that warp `warp` (0 or 1) tests; kept out of line so that its
-// registers do not add to the gather loops'.
+// Clustered samples among the 8 that warp `warp` (0 .. 7) tests, their loads in flight together (one
+// sample after the other took 25 us per launch); kept out of line so that its registers do not add to
+// the gather loops'.
 __device__ __noinline__ int ral_gather_votes(const GatherColumnsParams& P, int warp, int lane) {
-    int votes = 0;
-    for (int q = warp * 32; q < warp * 32 + 32; ++q) {
-        const ral_i64 at = (P.n_out - 32) / (kGatherSamples - 1) * q;
+    ral_u32 lo[kGatherSamples / 8], hi[kGatherSamples / 8];
+#pragma unroll
+    for (int q = 0; q < kGatherSamples / 8; ++q) {
+        const ral_i64 at = (P.n_out - 32) / (kGatherSamples - 1) * (warp * (kGatherSamples / 8) + q);
         const ral_i64 j = ral_index_at(P, at + lane);
-        const bool in = j >= 0 && j < P.n_in;
-        long long lo = in ? j : LLONG_MAX, hi = in ? j : LLONG_MIN;
-        for (int off = 16; off > 0; off >>= 1) {
-            lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, off));
-            hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, off));
-        }
-        votes += (hi < lo || hi - lo < kGatherClusterSpan) ? 1 : 0;
+        const bool in = j >= 0 && j < P.n_in;  // rows are 32-bit: an index inside the input fits
+        lo[q] = in ? (ral_u32)j : 0xffffffffu;
+        hi[q] = in ? (ral_u32)j : 0u;
+    }
+    int votes = 0;
+#pragma unroll
+    for (int q = 0; q < kGatherSamples / 8; ++q) {
+        const ral_u32 a = __reduce_min_sync(0xffffffffu, lo[q]), b = __reduce_max_sync(0xffffffffu, hi[q]);
+        votes += (b < a || b - a < kGatherClusterSpan) ? 1 : 0;
     }
     return votes;
 }
@@ -202,22 +206,24 @@ __device__ __noinline__ int ral_gather_votes(const GatherColumnsParams& P, int w
 // 48 registers, five resident blocks of 256 threads per SM (a bound of six spills registers in the
 // gather loops).
 __global__ void __launch_bounds__(256, 5) gather_columns_kernel(const __grid_constant__ GatherColumnsParams P) {
+    if (P.scattered && *P.scattered) return;
     __shared__ unsigned long long s_cnt[kMaxGatherColumns];
     __shared__ int s_clustered;
     for (int c = threadIdx.x; c < P.num_columns; c += blockDim.x) s_cnt[c] = 0;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    // the order: warps 0 and 1 each test 32 samples of 32 consecutive indices (the same samples in
-    // every block); a sample is clustered when its in-range indices span fewer than
+    // the order: each warp tests 8 samples of 32 consecutive indices (the same samples in every block); a
+    // sample is clustered when its in-range indices span fewer than
     // kGatherClusterSpan input rows; a launch is clustered when at least half its samples are
     if (threadIdx.x == 0) s_clustered = 0;
     __syncthreads();
-    if (P.num_columns > 1 && P.n_out >= 32 * kGatherSamples && warp < 2) {
+    if (!P.scattered && P.num_columns > 1 && P.n_out >= 32 * kGatherSamples) {
         const int votes = ral_gather_votes(P, warp, lane);
         if (lane == 0) atomicAdd(&s_clustered, votes);
     }
     __syncthreads();
-    const bool row_major = P.num_columns == 1 || P.n_out < 32 * kGatherSamples || 2 * s_clustered >= kGatherSamples;
+    const bool row_major =
+        P.scattered || P.num_columns == 1 || P.n_out < 32 * kGatherSamples || 2 * s_clustered >= kGatherSamples;
     const ral_i64 step_rows = 32 * kGatherRowsPerLane;
     const ral_i64 nsteps = (P.n_out + step_rows - 1) / step_rows;
     const ral_i64 gwarp = ((ral_i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -250,6 +256,16 @@ __global__ void __launch_bounds__(256, 5) gather_columns_kernel(const __grid_con
     if (P.valid_counts)
         for (int c = threadIdx.x; c < P.num_columns; c += blockDim.x)
             if (s_cnt[c]) atomicAdd(P.valid_counts + c, s_cnt[c]);
+}
+
+__global__ void __launch_bounds__(256) gather_probe_kernel(const __grid_constant__ GatherColumnsParams P, int32_t* scattered) {
+    __shared__ int s_votes;
+    if (threadIdx.x == 0) s_votes = 0;
+    __syncthreads();
+    const int votes = ral_gather_votes(P, threadIdx.x >> 5, threadIdx.x & 31);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_votes, votes);
+    __syncthreads();
+    if (threadIdx.x == 0) *scattered = 2 * s_votes >= kGatherSamples ? 0 : 1;
 }
 
 // ---- single-pass stream compaction (decoupled look-back) ---------------------------------
@@ -1340,6 +1356,13 @@ cudaError_t launch_gather_columns(const GatherColumnsParams& p, cudaStream_t st)
     const int64_t steps = (p.n_out + 32 * kGatherRowsPerLane - 1) / (32 * kGatherRowsPerLane);
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((steps + 7) / 8, (int64_t)sms * per_sm));
     gather_columns_kernel<<<(int)grid, 256, 0, st>>>(p);
+    note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gather_probe(const GatherColumnsParams& p, int32_t* scattered, cudaStream_t st) {
+    static_assert(kGatherProbeRows >= 32 * kGatherSamples, "a sample starts within the index");
+    gather_probe_kernel<<<1, 256, 0, st>>>(p, scattered);
     note_launch();
     return cudaGetLastError();
 }

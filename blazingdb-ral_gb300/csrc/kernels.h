@@ -40,12 +40,25 @@ struct GatherColumnsParams {
     unsigned long long* valid_counts;  // one counter per column with out_valid (zeroed), or null
     int32_t num_columns;
     int32_t idx_width;  // 1, 2, 4 or 8
+    // optional: nonzero where the index is scattered (launch_gather_probe), and another launch gathers the
+    // columns then
+    const int32_t* scattered;
 };
 
 // out_c[i] = in_c[idx[i]] for every column c, reading each index once; other indices leave
 // out_c[i] untouched.  Output validity words are built by ballot, 32 rows at a time, and their
 // set bits counted into valid_counts[c].
 cudaError_t launch_gather_columns(const GatherColumnsParams& p, cudaStream_t st);
+
+// *scattered = whether p's index jumps about the input (samples of it span many rows; p.n_out of at least
+// kGatherProbeRows).
+constexpr int64_t kGatherProbeRows = 2048;
+cudaError_t launch_gather_probe(const GatherColumnsParams& p, int32_t* scattered, cudaStream_t st);
+
+// Every column by way of row records in `scratch` (gather_records.cu), where the int32 flag at its start
+// is nonzero; nothing where it is zero.  p.n_in at least 1.
+size_t gather_records_bytes(const GatherColumnsParams& p);
+cudaError_t launch_gather_records(const GatherColumnsParams& p, void* scratch, cudaStream_t st);
 
 // ---- line index of a delimited text buffer (the text scan) ---------------------------------
 
