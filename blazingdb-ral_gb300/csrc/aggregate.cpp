@@ -222,7 +222,7 @@ int process_aggregate(gdf_column* const* frame, int n_cols, const char* query, g
         const int grid = launch_blocks(*k, s.threads, rows_per_block, n);
         const int64_t nwords = aggregate_scratch_words(S, grid);
         uint64_t* d = nullptr;
-        if (int e = check_cuda(cudaMallocAsync((void**)&d, (size_t)nwords * 8, st), "cudaMallocAsync")) return e;
+        if (int e = scratch_alloc((void**)&d, (size_t)nwords * 8, st)) return e;
         int rc = check_cuda(cudaMemsetAsync(d, 0, (size_t)nwords * 8, st), "cudaMemsetAsync");
         std::vector<uint64_t> slots(L.total, 0);
         slots[L.n_rows] = (uint64_t)n;

@@ -87,7 +87,7 @@ int count_nulls(gdf_column* col, cudaStream_t st) {
         return kSuccess;
     }
     unsigned long long* d = nullptr;
-    if (int e = check_cuda(cudaMallocAsync((void**)&d, sizeof(unsigned long long), st), "cudaMallocAsync")) return e;
+    if (int e = scratch_alloc((void**)&d, sizeof(unsigned long long), st)) return e;
     cudaMemsetAsync(d, 0, sizeof(unsigned long long), st);
     if (int e = check_cuda(launch_count_valid((const uint32_t*)col->valid, col->size, d, st), "count_valid")) return e;
     unsigned long long h = 0;
@@ -341,7 +341,7 @@ int ral_materialize_column(const gdf_column* input, gdf_column* output, const gd
         cudaStream_t st = cudaStreamPerThread;
         unsigned long long* d = nullptr;
         if (output->valid) {
-            if (int e = check_cuda(cudaMallocAsync((void**)&d, sizeof(unsigned long long), st), "cudaMallocAsync")) return e;
+            if (int e = scratch_alloc((void**)&d, sizeof(unsigned long long), st)) return e;
             cudaMemsetAsync(d, 0, sizeof(unsigned long long), st);
         }
         if (int e = check_cuda(launch_gather(w, input->data, (const uint32_t*)input->valid, input->size, row_indices->data, iw, n,
@@ -435,11 +435,7 @@ int ral_materialize_columns(const gdf_column* const* inputs, gdf_column* const* 
         std::vector<unsigned long long> h(num_columns > 0 ? num_columns : 1, 0);
         if (n > 0 && num_columns > 0) {
             unsigned long long* d = nullptr;
-            cudaMemPool_t pool = nullptr;
-            if (int e = scratch_pool(&pool)) return e;
-            if (int e = check_cuda(cudaMallocFromPoolAsync((void**)&d, sizeof(unsigned long long) * num_columns, pool, st),
-                                   "cudaMallocFromPoolAsync"))
-                return e;
+            if (int e = scratch_alloc((void**)&d, sizeof(unsigned long long) * num_columns, st)) return e;
             int rc = check_cuda(cudaMemsetAsync(d, 0, sizeof(unsigned long long) * num_columns, st), "cudaMemsetAsync");
             p.valid_counts = d;
             if (!rc) rc = gather_columns(p, st);
@@ -531,7 +527,7 @@ int ral_apply_boolean_mask(const gdf_column* stencil, gdf_column* out_indices, g
         cudaStream_t st = cudaStreamPerThread;
         const int64_t words = compact_scratch_words(n);
         unsigned long long* scratch = nullptr;
-        if (int e = check_cuda(cudaMallocAsync((void**)&scratch, (size_t)words * 8, st), "cudaMallocAsync")) return e;
+        if (int e = scratch_alloc((void**)&scratch, (size_t)words * 8, st)) return e;
         if (int e = check_cuda(cudaMemsetAsync(scratch, 0, (size_t)words * 8, st), "cudaMemsetAsync")) {
             cudaFreeAsync(scratch, st);
             return e;

@@ -109,8 +109,9 @@ void remap_to(gdf_column* c, const ral_category* merged) {
         if (!c->data) throw ParseError("string category column without data");
         cudaStream_t st = cudaStreamPerThread;
         int32_t* d = nullptr;
-        cudaError_t e = cudaMallocAsync((void**)&d, table.size() * sizeof(int32_t), st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(d, table.data(), table.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+        if (scratch_alloc((void**)&d, table.size() * sizeof(int32_t), st))
+            throw ParseError(std::string("remapping category codes: ") + last_error());
+        cudaError_t e = cudaMemcpyAsync(d, table.data(), table.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = launch_category_remap(static_cast<int32_t*>(c->data), c->size, d, (int32_t)table.size(), st);
         if (d) cudaFreeAsync(d, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);

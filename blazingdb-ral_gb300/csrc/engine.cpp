@@ -163,6 +163,12 @@ int scratch_pool(cudaMemPool_t* out) {
     return kSuccess;
 }
 
+int scratch_alloc(void** out, size_t bytes, cudaStream_t st) {
+    cudaMemPool_t pool = nullptr;
+    if (int e = scratch_pool(&pool)) return e;
+    return check_cuda(cudaMallocFromPoolAsync(out, std::max<size_t>(bytes, 8), pool, st), "cudaMallocFromPoolAsync");
+}
+
 int copy_lane(CopyLane*& out) {
     int dev = 0;
     if (int e = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return e;
@@ -378,8 +384,7 @@ int perform_operation(gdf_column* const* outputs, int n_out, gdf_column* const* 
     uint64_t* d_counts = nullptr;
     cudaStream_t st = opt.stream;
     if (want_counts) {
-        if (int e = check_cuda(cudaMallocAsync((void**)&d_counts, sizeof(uint64_t) * n_out, st), "cudaMallocAsync"))
-            return e;
+        if (int e = scratch_alloc((void**)&d_counts, sizeof(uint64_t) * n_out, st)) return e;
         if (int e = check_cuda(cudaMemsetAsync(d_counts, 0, sizeof(uint64_t) * n_out, st), "cudaMemsetAsync"))
             return e;
     }
@@ -501,14 +506,14 @@ int perform_operation_host(gdf_column* const* outputs, int n_out, gdf_column* co
         if (d_counts) cudaFreeAsync(d_counts, hs.s[0]);
         cudaStreamSynchronize(hs.s[0]);
     };
-    if ((rc = check_cuda(cudaMallocAsync((void**)&d_counts, sizeof(uint64_t) * n_out, hs.s[0]), "cudaMallocAsync")) ||
+    if ((rc = scratch_alloc((void**)&d_counts, sizeof(uint64_t) * n_out, hs.s[0])) ||
         (rc = check_cuda(cudaMemsetAsync(d_counts, 0, sizeof(uint64_t) * n_out, hs.s[0]), "cudaMemsetAsync"))) {
         release();
         return rc;
     }
     cudaEventRecord(hs.ready, hs.s[0]);
     for (int k = 0; k < 3; k++) {
-        if ((rc = check_cuda(cudaMallocAsync((void**)&area[k], per_slot, hs.s[k]), "cudaMallocAsync"))) {
+        if ((rc = scratch_alloc((void**)&area[k], per_slot, hs.s[k]))) {
             release();
             return rc;
         }

@@ -94,6 +94,10 @@ void keep_pool_memory();
 // calls have freed it keeps at most kScratchPoolKept bytes at a synchronisation.
 constexpr uint64_t kScratchPoolKept = (uint64_t)8 << 30;
 int scratch_pool(cudaMemPool_t* out);
+// Stream-ordered scratch of one call from that pool (freed with cudaFreeAsync).  The device's default
+// pool keeps nothing at a synchronisation unless the process asks it to, so that an allocation there
+// maps memory again on every call: about 130 us for eight bytes.
+int scratch_alloc(void** out, size_t bytes, cudaStream_t st);
 
 // The copy stream of the calling thread on the current device, with its events (made once, kept
 // for the thread's life): host-to-device copies issued on it overlap kernels on the caller's stream.

@@ -38,8 +38,7 @@ struct DeviceBuffer {
     }
     int alloc(size_t bytes, cudaStream_t s) {
         st = s;
-        if (bytes == 0) bytes = 8;
-        return check_cuda(cudaMallocAsync(&p, bytes, s), "cudaMallocAsync");
+        return scratch_alloc(&p, bytes, s);
     }
 };
 
