@@ -910,6 +910,16 @@ int ral_server_copy_result(ral_server* server, int64_t request_id, gdf_column* c
         std::vector<gdf_column> src(num_outputs);
         if (int e = server->s.result(request_id, src.data(), num_outputs)) return e;
         cudaStream_t st = cudaStreamPerThread;
+        CopyList list;
+        list.n = 0;
+        auto add = [&](const void* s, void* d, size_t bytes) -> int {
+            if (!bytes) return kSuccess;
+            list.job[list.n++] = CopyJob{(const uint8_t*)s, (uint8_t*)d, (int64_t)bytes};
+            if (list.n < kMaxCopyList) return kSuccess;
+            const cudaError_t e = launch_copy_list(list, st);
+            list.n = 0;
+            return check_cuda(e, "copy of a served result");
+        };
         for (int o = 0; o < num_outputs; o++) {
             gdf_column* d = out_columns[o];
             if (!d) return set_error(kInvalidArgument, "null out column");
@@ -917,12 +927,14 @@ int ral_server_copy_result(ral_server* server, int64_t request_id, gdf_column* c
             if ((d->valid != nullptr) != (src[o].valid != nullptr))
                 return set_error(kInvalidArgument, "out column mask presence differs from the query's");
             const size_t nb = (size_t)src[o].size * gdf_dtype_size(src[o].dtype);
-            if (nb) cudaMemcpyAsync(d->data, src[o].data, nb, cudaMemcpyDeviceToDevice, st);
-            if (src[o].valid && src[o].size)
-                cudaMemcpyAsync(d->valid, src[o].valid, ((size_t)src[o].size + 7) / 8, cudaMemcpyDeviceToDevice, st);
+            if (int e = add(src[o].data, d->data, nb)) return e;
+            if (src[o].valid)
+                if (int e = add(src[o].valid, d->valid, ((size_t)src[o].size + 7) / 8)) return e;
             d->size = src[o].size;
             d->null_count = src[o].null_count;
         }
+        if (list.n)
+            if (int e = check_cuda(launch_copy_list(list, st), "copy of a served result")) return e;
         return check_cuda(cudaStreamSynchronize(st), "copy of a served result");
     });
 }

@@ -1378,21 +1378,61 @@ cudaError_t launch_parquet_level_lengths(const ParquetDecodeParams& p, cudaStrea
 
 // One block per job: bytes [src, src + bytes) to dst (16-byte loads and stores where both sides
 // share an alignment, single bytes otherwise).
-__global__ void __launch_bounds__(256) copy_jobs_kernel(const CopyJob* __restrict__ jobs, int32_t n_jobs) {
-    const CopyJob j = jobs[blockIdx.x];
+// One copy by threads t, t + step, ...: 16-byte words where source and destination agree in alignment.
+__device__ __forceinline__ void ral_copy(const CopyJob& j, int64_t t, int64_t step) {
     const uintptr_t s = (uintptr_t)j.src, d = (uintptr_t)j.dst;
     if (((s ^ d) & 15) == 0) {
         const int64_t lead = (int64_t)((16 - (s & 15)) & 15);
         const int64_t head = j.bytes < lead ? j.bytes : lead;
-        for (int64_t i = threadIdx.x; i < head; i += blockDim.x) j.dst[i] = j.src[i];
+        for (int64_t i = t; i < head; i += step) j.dst[i] = j.src[i];
         const int64_t nv = (j.bytes - head) >> 4;
         const uint4* sv = reinterpret_cast<const uint4*>(j.src + head);
         uint4* dv = reinterpret_cast<uint4*>(j.dst + head);
-        for (int64_t i = threadIdx.x; i < nv; i += blockDim.x) dv[i] = sv[i];
-        for (int64_t i = head + nv * 16 + threadIdx.x; i < j.bytes; i += blockDim.x) j.dst[i] = j.src[i];
+        for (int64_t i = t; i < nv; i += step) dv[i] = sv[i];
+        for (int64_t i = head + nv * 16 + t; i < j.bytes; i += step) j.dst[i] = j.src[i];
+    } else if (((s ^ d) & 3) == 0) {
+        const int64_t lead = (int64_t)((4 - (s & 3)) & 3);
+        const int64_t head = j.bytes < lead ? j.bytes : lead;
+        for (int64_t i = t; i < head; i += step) j.dst[i] = j.src[i];
+        const int64_t nv = (j.bytes - head) >> 2;
+        const ral_u32* sv = reinterpret_cast<const ral_u32*>(j.src + head);
+        ral_u32* dv = reinterpret_cast<ral_u32*>(j.dst + head);
+        for (int64_t i = t; i < nv; i += step) dv[i] = sv[i];
+        for (int64_t i = head + nv * 4 + t; i < j.bytes; i += step) j.dst[i] = j.src[i];
     } else {
-        for (int64_t i = threadIdx.x; i < j.bytes; i += blockDim.x) j.dst[i] = j.src[i];
+        for (int64_t i = t; i < j.bytes; i += step) j.dst[i] = j.src[i];
     }
+}
+
+__global__ void __launch_bounds__(256) copy_jobs_kernel(const CopyJob* __restrict__ jobs, int32_t n_jobs) {
+    ral_copy(jobs[blockIdx.x], threadIdx.x, blockDim.x);
+}
+
+__global__ void __launch_bounds__(256) copy_list_kernel(const __grid_constant__ CopyList list) {
+    ral_copy(list.job[blockIdx.y], (int64_t)blockIdx.x * 256 + threadIdx.x, (int64_t)gridDim.x * 256);
+}
+
+cudaError_t launch_copy_list(const CopyList& list, cudaStream_t st) {
+    int64_t most = 0;
+    for (int k = 0; k < list.n; k++) most = std::max(most, list.job[k].bytes);
+    if (most <= 0) return cudaSuccess;
+    // 4 of the 16-byte words a thread, up to the device's threads for all jobs together
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((most + 16383) / 16384, (152 * 8 + list.n - 1) / list.n));
+    copy_list_kernel<<<dim3((unsigned)blocks, (unsigned)list.n), 256, 0, st>>>(list);
+    note_launch();
+    return cudaGetLastError();
+}
+
+__global__ void __launch_bounds__(96) copy_headers_kernel(const HeaderJob* __restrict__ jobs, unsigned long long* __restrict__ dst) {
+    const HeaderJob j = jobs[blockIdx.x];
+    if ((int64_t)threadIdx.x < j.words) dst[(size_t)blockIdx.x * 67 + threadIdx.x] = __ldcg(j.src + threadIdx.x);
+}
+
+cudaError_t launch_copy_headers(const HeaderJob* jobs, int32_t n, unsigned long long* dst, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    copy_headers_kernel<<<n, 96, 0, st>>>(jobs, dst);
+    note_launch();
+    return cudaGetLastError();
 }
 
 cudaError_t launch_copy_jobs(const CopyJob* jobs, int32_t n_jobs, cudaStream_t st) {

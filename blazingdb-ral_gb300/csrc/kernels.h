@@ -144,6 +144,22 @@ struct CopyJob {
 };
 cudaError_t launch_copy_jobs(const CopyJob* jobs, int32_t n_jobs, cudaStream_t st);
 
+// The same for large buffers, by value, each spread over the device: one launch in place of a copy each
+// (the outputs of a served result, 4 copies and their wait: 30 us).
+constexpr int kMaxCopyList = 128;
+struct CopyList {
+    CopyJob job[kMaxCopyList];
+    int32_t n;
+};
+cudaError_t launch_copy_list(const CopyList& list, cudaStream_t st);
+// words[k] (at most 67) 8-byte words from src[k], device memory, to dst + 67 k, page-locked host memory: the
+// finished requests' headers of a served wave, one launch in place of a copy each.
+struct HeaderJob {
+    const unsigned long long* src;
+    int64_t words;
+};
+cudaError_t launch_copy_headers(const HeaderJob* jobs, int32_t n, unsigned long long* dst, cudaStream_t st);
+
 // Pages of [page_lo, page_hi) whose level length is -1 (Snappy v1 pages): the length from the
 // first 4 bytes of their decompressed data, and their values' offset after it.
 cudaError_t launch_parquet_level_lengths(const ParquetDecodeParams& p, cudaStream_t st);

@@ -14,6 +14,7 @@
 
 #include "batch.h"
 #include "engine.h"
+#include "kernels.h"
 
 namespace ral {
 
@@ -26,14 +27,15 @@ size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 constexpr double kAgeRowsPerSecond = 1e10;
 
 // Item shape of a query: vector width from the widest column, chunks of RAL_SERVER_CHUNK rows
-// (default 2048; 1024 measured the same), predicate unroll 2, and the FP64 instructions
-// (RAL_SERVER_SOFT_FP=1 for the integer-pipe double operations: measured 1656 requests/s at
-// capacity against 1756 with the FP64 instructions).
+// (default 512: a burst of 16 requests over tables of up to 4M rows took 920 / 840 / 795 us at 2048 / 1024 /
+// 512 rows, p50 at 3470 requests/s 3.07 / 2.12 / 1.91 ms; 256 was slower, capacity is the same), predicate
+// unroll 2, and the FP64 instructions (RAL_SERVER_SOFT_FP=1 for the integer-pipe double operations:
+// measured 1656 requests/s at capacity against 1756 with the FP64 instructions).
 Shape query_shape(const FilterPlan& plan, bool aligned16) {
     Shape sh;
     sh.G = aligned16 ? 16 / filter_max_width(plan.spec) : 1;
     const char* c = std::getenv("RAL_SERVER_CHUNK");
-    const int rows = c && std::atoi(c) >= 32 && std::atoi(c) <= 8192 ? std::atoi(c) : 2048;
+    const int rows = c && std::atoi(c) >= 32 && std::atoi(c) <= 8192 ? std::atoi(c) : 512;
     sh.J = std::max(1, rows / (32 * sh.G));
     sh.threads = 256;
     sh.min_blocks = 1;
@@ -287,10 +289,10 @@ int Server::ensure_linked() {
     stride_ = stride;
     smem_words_ = smem;
     linked_queries_ = (int)queries_.size();
-    // wave buffers: descs | prefix | base | fn | counter
+    // wave buffers: descs | prefix | base | fn | headers | counter
     const size_t M = (size_t)max_wave_requests_;
-    const size_t bytes =
-        round_up(M * stride_ * 8, 16) + round_up((M + 1) * 8, 16) + round_up(M * 8, 16) + round_up(M * 4, 16) + 16;
+    const size_t bytes = round_up(M * stride_ * 8, 16) + round_up((M + 1) * 8, 16) + round_up(M * 8, 16) +
+                         round_up(M * 4, 16) + M * sizeof(HeaderJob) + 16;
     if (waves_.empty()) waves_.resize(max_waves_);
     for (auto& w : waves_) {
         if (!w.stream && check_cuda(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking), "cudaStreamCreate"))
@@ -365,13 +367,17 @@ int Server::submit(int query_id, bool keep, int64_t* request_id) {
 
 int Server::launch_wave(Wave& w, const std::vector<int64_t>& reqs, const std::vector<int64_t>& take) {
     const int NP = (int)reqs.size();
-    const size_t M = (size_t)max_wave_requests_;
+    // this wave's arrays back to back: one copy
+    const size_t M = (size_t)NP;
     char* h = (char*)w.h_desc;
     uint64_t* descs = (uint64_t*)h;
     const size_t off_prefix = round_up(M * stride_ * 8, 16);
     const size_t off_base = off_prefix + round_up((M + 1) * 8, 16);
     const size_t off_fn = off_base + round_up(M * 8, 16);
-    const size_t off_counter = off_fn + round_up(M * 4, 16);
+    const size_t off_heads = off_fn + round_up(M * 4, 16);
+    const size_t off_counter = off_heads + M * sizeof(HeaderJob);
+    HeaderJob* heads = (HeaderJob*)(h + off_heads);
+    bool any_last = false;
     long long* prefix = (long long*)(h + off_prefix);
     long long* base = (long long*)(h + off_base);
     int* fn = (int*)(h + off_fn);
@@ -399,15 +405,15 @@ int Server::launch_wave(Wave& w, const std::vector<int64_t>& reqs, const std::ve
         fn[k] = q.fn;
         r.next_chunk += take[k];
         w.last[k] = r.next_chunk >= q.chunks;
+        any_last |= w.last[k] != 0;
+        // scratch headers of the requests that finish in this wave: error flag, kept rows, valid counts
+        heads[k].src = (const unsigned long long*)r.scratch;
+        heads[k].words = w.last[k] ? filter_scratch_header((int)q.plan->out_dtypes.size()) : 0;
         r.in_wave = true;
     }
     const long long total = prefix[NP];
     char* d = (char*)w.d_desc;
-    cudaMemcpyAsync(d, h, (size_t)NP * stride_ * 8, cudaMemcpyHostToDevice, w.stream);
-    cudaMemcpyAsync(d + off_prefix, h + off_prefix, (size_t)(NP + 1) * 8, cudaMemcpyHostToDevice, w.stream);
-    cudaMemcpyAsync(d + off_base, h + off_base, (size_t)NP * 8, cudaMemcpyHostToDevice, w.stream);
-    cudaMemcpyAsync(d + off_fn, h + off_fn, (size_t)NP * 4, cudaMemcpyHostToDevice, w.stream);
-    cudaMemcpyAsync(d + off_counter, h + off_counter, 16, cudaMemcpyHostToDevice, w.stream);
+    cudaMemcpyAsync(d, h, off_counter + 16, cudaMemcpyHostToDevice, w.stream);
     const void* a_descs = d;
     int a_stride = stride_;
     const void* a_prefix = d + off_prefix;
@@ -425,15 +431,10 @@ int Server::launch_wave(Wave& w, const std::vector<int64_t>& reqs, const std::ve
             return e;
         note_launch();
     }
-    // scratch headers of the requests that finish in this wave: error flag, kept rows, valid counts
-    uint64_t* hh = (uint64_t*)w.h_head;
-    for (int k = 0; k < NP; k++) {
-        if (!w.last[k]) continue;
-        ServerRequest& r = *requests_[reqs[k]];
-        const int NO = (int)queries_[r.query]->plan->out_dtypes.size();
-        cudaMemcpyAsync(hh + (size_t)k * 67, r.scratch, (size_t)filter_scratch_header(NO) * 8, cudaMemcpyDeviceToHost,
-                        w.stream);
-    }
+    if (any_last)
+        if (int e = check_cuda(launch_copy_headers((const HeaderJob*)(d + off_heads), NP, (unsigned long long*)w.h_head, w.stream),
+                               "copy of the requests' headers"))
+            return e;
     if (int e = check_cuda(cudaEventRecord(w.done, w.stream), "cudaEventRecord")) return e;
     w.reqs = reqs;
     w.take = take;
