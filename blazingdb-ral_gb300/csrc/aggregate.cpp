@@ -19,8 +19,8 @@
 //   * SUM / MIN / MAX of an empty input, or of a bare input whose rows are all null, are null
 //     scalars; AVG is null for an empty or all-null input, else the SUM as double divided by the
 //     count (GroupBy.cpp:256-277);
-//   * integer sums wrap in int64; float sums are exact IEEE adds in a fixed order (per thread,
-//     then warps, blocks and block partials in index order), so a result does not change between
+//   * integer sums wrap in int64; float sums are IEEE adds in a fixed order (per thread,
+//     then trees over lanes, warps and the blocks' partials), so a result does not change between
 //     calls on the same GPU, but is not the bits of any one sequential order.
 #include <cuda_runtime.h>
 
