@@ -135,16 +135,21 @@ struct SnappyJob {
 // One warp per job; a malformed stream or a length mismatch adds one to *status.
 cudaError_t launch_snappy_decompress(const SnappyJob* jobs, int32_t n_jobs, unsigned long long* status, cudaStream_t st);
 
-// Byte copies gathered into one launch (one block per job): small pieces of a page-locked file
-// (dictionaries) brought into device memory.
+// Byte copies and fills gathered into one launch (one block per job of some 16 KiB): what a Parquet scan
+// needs before its pages are decoded.
 struct CopyJob {
     const uint8_t* src;
     uint8_t* dst;
     int64_t bytes;
 };
-cudaError_t launch_copy_jobs(const CopyJob* jobs, int32_t n_jobs, cudaStream_t st);
+struct PrepareJob {
+    CopyJob copy;           // src null: every byte becomes `fill`
+    int32_t fill;
+    int32_t pad;
+};
+cudaError_t launch_prepare_jobs(const PrepareJob* jobs, int32_t n_jobs, cudaStream_t st);
 
-// The same for large buffers, by value, each spread over the device: one launch in place of a copy each
+// Copies of large buffers, by value, each spread over the device: one launch in place of a copy each
 // (the outputs of a served result, 4 copies and their wait: 30 us).
 constexpr int kMaxCopyList = 128;
 struct CopyList {

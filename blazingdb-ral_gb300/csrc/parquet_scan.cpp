@@ -5,8 +5,9 @@
 // (src/io/data_parser/ParquetParser.cpp:36-90, cudf's Parquet reader), and a LogicalFilter above
 // it evaluates its condition over the scanned frame and compacts it (CalciteInterpreter.cpp:509).
 // Here the footer and page headers are read on the host (parquet_meta.cpp) and the pages are
-// decoded on the device: a page-locked file is read in place over the host link, other host memory
-// is copied in, column chunk by column chunk, in batches decoded while the next batch is copied.
+// decoded on the device: a file whose memory the device can read is read in place over the host link,
+// other host memory is copied in, column chunk by column chunk, in batches decoded while the next batch
+// is copied.
 // Snappy-compressed pages are decompressed first (one warp per page), then a levels kernel decodes
 // optional pages' definition levels, a dictionary kernel the indices of dictionary-encoded pages,
 // and a values kernel every page's values in 8192-row items; the fused filter kernel (filter.cpp)
@@ -16,12 +17,12 @@
 // uncompressed or Snappy-compressed chunks.  Anything else (other codecs, encodings or types,
 // nested schemas) is refused with RAL_ERROR_UNSUPPORTED.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
-#include <map>
-#include <memory>
 #include <string>
 #include <vector>
 
@@ -55,8 +56,35 @@ int64_t batch_bytes() {
     return v > 0 ? (int64_t)v : ((int64_t)24 << 20);
 }
 
-// The address kernels read file[0, n) at when it is page-locked (or mapped) host memory of this
-// process, else null.  Both ends are checked: a registered range covers the whole buffer.
+// Whether the device reads ordinary host memory through the host's own page tables (it is coherent with
+// the CPU over the link), as fast as page-locked memory.
+bool reads_host_pages() {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return v != 0;
+}
+
+// Whether eight pages spread over file[0, n) are all in memory (3 us).  A mapped file that has not been read
+// yet would come in by a fault of the device per page: it is copied in, which reads it in order.
+bool resident(const uint8_t* file, int64_t n) {
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    for (int64_t k = 0; k < 8; k++) {
+        const uintptr_t at = ((uintptr_t)file + (uintptr_t)((n - 1) / 7 * k + (n - 1) % 7 * k / 7)) & ~(page - 1);
+        unsigned char in = 0;
+        if (mincore((void*)at, 1, &in) != 0 || !(in & 1)) return false;
+    }
+    return true;
+}
+
+// The address kernels read file[0, n) at, or null where the chunks are to be copied in: page-locked (or
+// mapped) host memory of this process, and, where the device reads them at the link's rate too, ordinary
+// pages.  A copy from those returns when it is done, so nothing overlapped it: 700,001 rows of dictionary
+// pages with nulls 260 us copied, 226 in place; 6M rows of PLAIN pages 1365 and 1021; 10,000 rows 108
+// and 100.  Both ends are checked: a registered range covers the whole buffer.
 const uint8_t* device_view(const uint8_t* file, int64_t n) {
     if (std::getenv("RAL_PARQUET_STAGED")) return nullptr;  // always copy the chunks in
     cudaPointerAttributes a{}, b{};
@@ -64,6 +92,8 @@ const uint8_t* device_view(const uint8_t* file, int64_t n) {
         cudaGetLastError();
         return nullptr;
     }
+    if (a.type == cudaMemoryTypeUnregistered && b.type == cudaMemoryTypeUnregistered)
+        return reads_host_pages() && resident(file, n) ? file : nullptr;
     if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer) return nullptr;
     if ((const uint8_t*)b.devicePointer != (const uint8_t*)a.devicePointer + (n - 1)) return nullptr;
     return (const uint8_t*)a.devicePointer;
@@ -245,6 +275,41 @@ int plan_chunks(const uint8_t* file, int64_t n, const pq::FileMeta& meta, const 
     return kSuccess;
 }
 
+// Chunks copied from the file to `to` in batches of about batch_bytes(), each batch's copies on the copy
+// lane's stream while the batch before it is decoded on `st`.
+template <typename Decode>
+int decode_copied(const uint8_t* file, const ChunkPlan& plan, uint8_t* to, cudaStream_t st, Decode&& decode) {
+    CopyLane* lane = nullptr;
+    if (int e = copy_lane(lane)) return e;
+    // the copy lane starts after this stream's work so far; on every exit this stream waits for
+    // the lane before any buffer is freed
+    if (int e = check_cuda(cudaEventRecord(lane->ready, st), "cudaEventRecord")) return e;
+    if (int e = check_cuda(cudaStreamWaitEvent(lane->s, lane->ready, 0), "cudaStreamWaitEvent")) return e;
+    LaneJoin join{lane, st};
+    const int64_t batch_size = batch_bytes();
+    size_t batch = 0;
+    for (size_t c0 = 0; c0 < plan.chunks.size(); batch++) {
+        size_t c1 = c0;
+        int64_t bytes = 0;
+        while (c1 < plan.chunks.size() && (c1 == c0 || bytes < batch_size)) {
+            const Chunk& c = plan.chunks[c1];
+            if (c.bytes > 0 && check_cuda(cudaMemcpyAsync(to + c.dev_off, file + c.file_off, (size_t)c.bytes,
+                                                          cudaMemcpyHostToDevice, lane->s),
+                                          "cudaMemcpyAsync"))
+                return kCudaError;
+            bytes += c.bytes;
+            c1++;
+        }
+        cudaEvent_t copied = nullptr;
+        if (int e = lane_event(*lane, batch, &copied)) return e;
+        if (int e = check_cuda(cudaEventRecord(copied, lane->s), "cudaEventRecord")) return e;
+        if (int e = check_cuda(cudaStreamWaitEvent(st, copied, 0), "cudaStreamWaitEvent")) return e;
+        if (int e = decode(c0, c1)) return e;
+        c0 = c1;
+    }
+    return kSuccess;
+}
+
 }  // namespace
 
 int parquet_schema(const uint8_t* file, int64_t n, int64_t* rows, int32_t* n_columns, int32_t* dtypes, int32_t capacity) {
@@ -291,127 +356,132 @@ int parquet_scan_filter(const uint8_t* file, int64_t n, const int32_t* projectio
 
     cudaStream_t st = cudaStreamPerThread;
     keep_pool_memory();
-    CopyLane* lane = nullptr;
-    if (int e = copy_lane(lane)) return e;
-    DevBuf dfile(st), dunpack(st), djobs(st), dpages(st), dstatus(st), ditems(st), dpresent(st), didx(st);
-    // decoded columns: the outputs themselves without a filter, a frame of temporaries with one
-    std::vector<std::unique_ptr<DevBuf>> owned;
+    // The kernels read the file where it lies (over the host link, no staging copy) where they can; else
+    // it is copied in, chunk by chunk.  Chunks with dictionary-encoded pages that are not decompressed are
+    // copied to device memory by a kernel even then: dictionaries are looked up at random, and the walk of
+    // the indices' run headers waits for every read (runs of 504 values: 325 us copied, 468 in place).  Snappy pages are decompressed into the unpack buffer.
+    const uint8_t* direct = device_view(file, n);
+    std::vector<int64_t> copied(plan.chunks.size(), -1);  // in place: where a chunk that is copied goes
+    int64_t file_bytes = direct ? 0 : plan.packed;
+    if (direct) {
+        for (size_t k = 0; k < pages.size(); k++) {
+            if (pages[k].dict_count <= 0 || (plan.where[k].unpack >= 0 && plan.dict_where[k].unpack >= 0)) continue;
+            const Chunk& c = plan.chunks[plan.where[k].chunk];
+            int64_t& at = copied[plan.where[k].chunk];
+            if (at >= 0) continue;
+            // the copy keeps the source's offset within 16 bytes, so that it moves whole 16-byte words
+            at = file_bytes + (int64_t)((uintptr_t)(direct + c.file_off) & 15);
+            file_bytes = ((at + c.bytes + 15) & ~15ll) + 16;
+        }
+    }
+    // One device buffer: the decoded columns (the outputs themselves without a filter), the counters that
+    // start at zero, the tables, dictionary indices, decompressed pages, copied chunks.
+    int64_t arena_bytes = 0;
+    auto place = [&](int64_t bytes) {
+        const int64_t at = arena_bytes;
+        arena_bytes += (std::max<int64_t>(bytes, 16) + 255) & ~255ll;
+        return at;
+    };
+    const int64_t mbytes = (int64_t)gdf_valid_allocation_size(std::max<int64_t>(rows, 1));
+    std::vector<int64_t> frame_at(n_proj), mask_at(n_proj);
+    if (filter_q)
+        for (int q = 0; q < n_proj; q++) {
+            frame_at[q] = place(rows * gdf_dtype_size(dtypes[q]));
+            mask_at[q] = place(mbytes);
+        }
+    // status, items, present rows
+    const int64_t zero_bytes = (1 + n_proj) * 8 + items * 4 + (int64_t)pages.size() * 4;
+    const int64_t zero_at = place(zero_bytes);
+    const int64_t idx_at = place(plan.n_idx * 4);
+    const int64_t unpack_at = place(plan.unpack_bytes);
+    const int64_t file_at0 = place(file_bytes);
+    // the fills and copies before the decode, in pieces of at least kPrepareBytes
+    std::vector<PrepareJob> prep;
+    const int64_t kPrepareBytes = 16384;
+    int64_t prep_bytes = zero_bytes + n_proj * mbytes;
+    for (size_t c = 0; c < copied.size(); c++)
+        if (copied[c] >= 0) prep_bytes += plan.chunks[c].bytes;
+    const int64_t piece = std::max<int64_t>(kPrepareBytes, (prep_bytes / 8192 + 15) & ~15ll);
+    const int64_t tables_at = place(0);  // the last: its size follows from the jobs
+    const int64_t max_jobs = prep_bytes / piece + 2 + 3 * n_proj + (int64_t)plan.chunks.size();
+    const int64_t tables_bytes = max_jobs * (int64_t)sizeof(PrepareJob) + (int64_t)plan.unpacks.size() * (int64_t)sizeof(SnappyJob) +
+                                 (int64_t)pages.size() * (int64_t)sizeof(ParquetPage);
+    DevBuf arena(st);
+    if (int e = arena.alloc((size_t)(tables_at + tables_bytes))) return e;
+    uint8_t* const base = (uint8_t*)arena.p;
+    auto job = [&](const uint8_t* src, uint8_t* dst, int64_t bytes, int fill) {
+        for (int64_t o = 0; o < bytes; o += piece)
+            prep.push_back({{src ? src + o : nullptr, dst + o, std::min(piece, bytes - o)}, fill, 0});
+    };
     std::vector<gdf_column> frame(n_proj);
     std::vector<gdf_column*> pframe(n_proj);
     for (int q = 0; q < n_proj; q++) {
         frame[q] = gdf_column{};
         frame[q].dtype = dtypes[q];
         frame[q].size = (gdf_size_type)rows;
-        if (filter_q) {
-            owned.emplace_back(new DevBuf(st));
-            if (int e = owned.back()->alloc((size_t)rows * gdf_dtype_size(dtypes[q]) + gdf_valid_allocation_size(rows)))
-                return e;
-            frame[q].data = owned.back()->p;
-            frame[q].valid = (gdf_valid_type*)((char*)owned.back()->p + (size_t)rows * gdf_dtype_size(dtypes[q]));
-            // a multiple of 16 bytes keeps the mask 4-byte aligned
-            if (((uintptr_t)frame[q].valid) & 3) return set_error(kInvalidArgument, "internal: unaligned mask");
-        } else {
-            frame[q].data = outs[q]->data;
-            frame[q].valid = outs[q]->valid;
-        }
+        frame[q].data = filter_q ? (void*)(base + frame_at[q]) : outs[q]->data;
+        frame[q].valid = filter_q ? (gdf_valid_type*)(base + mask_at[q]) : outs[q]->valid;
         pframe[q] = &frame[q];
         // a required column's rows are all present; an optional column's bits are set by the levels
-        const size_t mbytes = gdf_valid_allocation_size(std::max<int64_t>(rows, 1));
-        cudaMemsetAsync(frame[q].valid, 0, mbytes, st);
-        if (!optional[q] && rows > 0) {
-            if (rows >= 8) cudaMemsetAsync(frame[q].valid, 0xff, (size_t)(rows / 8), st);
-            if (rows % 8) cudaMemsetAsync((char*)frame[q].valid + rows / 8, (1 << (rows % 8)) - 1, 1, st);
-        }
+        uint8_t* const m = (uint8_t*)frame[q].valid;
+        const int64_t full = optional[q] ? 0 : rows / 8, part = optional[q] ? 0 : rows % 8;
+        job(nullptr, m, full, 0xff);
+        if (part) job(nullptr, m + full, 1, (1 << part) - 1);
+        job(nullptr, m + full + (part ? 1 : 0), mbytes - full - (part ? 1 : 0), 0);
     }
-    // A page-locked file is read by the kernels where it lies (over the host link, no staging copy);
-    // any other host memory is copied in, chunk by chunk.  Snappy pages are decompressed into the
-    // unpack buffer first.
-    const uint8_t* direct = device_view(file, n);
-    if (!direct)
-        if (int e = dfile.alloc((size_t)plan.packed)) return e;
-    if (int e = dunpack.alloc((size_t)plan.unpack_bytes)) return e;
+    job(nullptr, base + zero_at, zero_bytes, 0);
+    for (size_t c = 0; c < copied.size(); c++)
+        if (copied[c] >= 0)
+            job(direct + plan.chunks[c].file_off, base + file_at0 + copied[c], plan.chunks[c].bytes, 0);
     auto file_at = [&](int64_t off, int32_t chunk) -> const uint8_t* {
-        if (direct) return direct + off;
         const Chunk& c = plan.chunks[chunk];
-        return (const uint8_t*)dfile.p + c.dev_off + (off - c.file_off);
+        if (direct && copied[chunk] < 0) return direct + off;
+        return base + file_at0 + (direct ? copied[chunk] : c.dev_off) + (off - c.file_off);
     };
     auto where_at = [&](const PageWhere& w) -> const uint8_t* {
-        return w.unpack >= 0 ? (const uint8_t*)dunpack.p + w.unpack : file_at(w.file_off, w.chunk);
+        return w.unpack >= 0 ? base + unpack_at + w.unpack : file_at(w.file_off, w.chunk);
     };
-    // read in place, a dictionary would be looked up at random over the host link: the
-    // dictionaries come into device memory first (one small copy job each, one launch)
-    DevBuf ddict(st), dcopies(st);
-    std::map<int64_t, int64_t> dict_copy;  // a dictionary's file offset -> its offset in ddict
-    std::vector<CopyJob> cjobs;
-    if (direct) {
-        int64_t dbytes = 0;
-        for (size_t k = 0; k < pages.size(); k++) {
-            const PageWhere& dw = plan.dict_where[k];
-            if (pages[k].dict_count <= 0 || dw.unpack >= 0 || dict_copy.count(dw.file_off)) continue;
-            // the copy keeps the source's offset within 16 bytes, so that it moves whole 16-byte words
-            const int64_t mis = (int64_t)((uintptr_t)(direct + dw.file_off) & 15);
-            dict_copy[dw.file_off] = dbytes + mis;
-            const int64_t b = (int64_t)pages[k].dict_count * gdf_dtype_size(dtypes[pages[k].column]);
-            cjobs.push_back({direct + dw.file_off, nullptr, b});
-            dbytes += ((mis + b + 15) & ~15ll) + 16;
-        }
-        if (!cjobs.empty()) {
-            if (int e = ddict.alloc((size_t)dbytes)) return e;
-            for (size_t k = 0; k < pages.size(); k++) {
-                const PageWhere& dw = plan.dict_where[k];
-                if (pages[k].dict_count <= 0 || dw.unpack >= 0) continue;
-                pages[k].dict = (int64_t)(uintptr_t)((char*)ddict.p + dict_copy[dw.file_off]);
-            }
-            for (CopyJob& cj : cjobs) {
-                const int64_t off = (int64_t)(cj.src - direct);
-                cj.dst = (uint8_t*)ddict.p + dict_copy[off];
-            }
-            if (int e = dcopies.alloc(cjobs.size() * sizeof(CopyJob))) return e;
-            if (int e = check_cuda(cudaMemcpyAsync(dcopies.p, cjobs.data(), cjobs.size() * sizeof(CopyJob),
-                                                   cudaMemcpyHostToDevice, st),
-                                   "cudaMemcpyAsync"))
-                return e;
-            if (int e = check_cuda(launch_copy_jobs((const CopyJob*)dcopies.p, (int32_t)cjobs.size(), st), "dictionary copies"))
-                return e;
-        }
-    }
     for (size_t k = 0; k < pages.size(); k++) {
         pages[k].data = (int64_t)(uintptr_t)where_at(plan.where[k]);
-        if (pages[k].dict_count > 0 && !(direct && plan.dict_where[k].unpack < 0))
-            pages[k].dict = (int64_t)(uintptr_t)where_at(plan.dict_where[k]);
+        if (pages[k].dict_count > 0) pages[k].dict = (int64_t)(uintptr_t)where_at(plan.dict_where[k]);
     }
     std::vector<SnappyJob> jobs(plan.unpacks.size());
     for (size_t k = 0; k < jobs.size(); k++) {
         const Unpack& u = plan.unpacks[k];
         jobs[k].src = file_at(u.src_off, u.chunk);
-        jobs[k].dst = (uint8_t*)dunpack.p + u.dst_off;
+        jobs[k].dst = base + unpack_at + u.dst_off;
         jobs[k].src_bytes = (int32_t)u.src_bytes;
         jobs[k].dst_bytes = (int32_t)u.dst_bytes;
         jobs[k].prefix = u.prefix;
     }
-    if (int e = djobs.alloc(jobs.size() * sizeof(SnappyJob))) return e;
-    if (!jobs.empty() && check_cuda(cudaMemcpyAsync(djobs.p, jobs.data(), jobs.size() * sizeof(SnappyJob),
-                                                    cudaMemcpyHostToDevice, st),
-                                    "cudaMemcpyAsync"))
-        return kCudaError;
-    if (int e = dpages.alloc(pages.size() * sizeof(ParquetPage))) return e;
-    if (!pages.empty() &&
-        check_cuda(cudaMemcpyAsync(dpages.p, pages.data(), pages.size() * sizeof(ParquetPage), cudaMemcpyHostToDevice, st),
-                   "cudaMemcpyAsync"))
-        return kCudaError;
-    if (int e = dstatus.alloc((size_t)(1 + n_proj) * 8)) return e;
-    cudaMemsetAsync(dstatus.p, 0, (size_t)(1 + n_proj) * 8, st);
-    if (int e = ditems.alloc((size_t)items * 4)) return e;
-    cudaMemsetAsync(ditems.p, 0, (size_t)items * 4, st);
-    if (int e = dpresent.alloc(pages.size() * 4)) return e;
-    cudaMemsetAsync(dpresent.p, 0, pages.size() * 4, st);
-    if (int e = didx.alloc((size_t)plan.n_idx * 4)) return e;
+    // the tables, in one copy
+    std::vector<uint8_t> tables(prep.size() * sizeof(PrepareJob) + jobs.size() * sizeof(SnappyJob) + pages.size() * sizeof(ParquetPage));
+    uint8_t* const djobs = base + tables_at + prep.size() * sizeof(PrepareJob);
+    uint8_t* const dpages = djobs + jobs.size() * sizeof(SnappyJob);
+    if (!prep.empty()) std::memcpy(tables.data(), prep.data(), prep.size() * sizeof(PrepareJob));
+    if (!jobs.empty()) std::memcpy(tables.data() + (djobs - base - tables_at), jobs.data(), jobs.size() * sizeof(SnappyJob));
+    if (!pages.empty()) std::memcpy(tables.data() + (dpages - base - tables_at), pages.data(), pages.size() * sizeof(ParquetPage));
+    if ((int64_t)tables.size() > tables_bytes) return set_error(kInvalidArgument, "internal: more preparation jobs than planned");
+    // before the call returns, nothing reads the caller's file any more
+    struct Drain {
+        cudaStream_t st;
+        bool on;
+        ~Drain() {
+            if (on) cudaStreamSynchronize(st);
+        }
+    } drain{st, direct != nullptr};
+    if (int e = check_cuda(cudaMemcpyAsync(base + tables_at, tables.data(), tables.size(), cudaMemcpyHostToDevice, st),
+                           "cudaMemcpyAsync"))
+        return e;
+    if (int e = check_cuda(launch_prepare_jobs((const PrepareJob*)(base + tables_at), (int32_t)prep.size(), st),
+                           "Parquet preparation"))
+        return e;
     ParquetDecodeParams dp{};
-    dp.pages = (ParquetPage*)dpages.p;
-    dp.status = (unsigned long long*)dstatus.p;
-    dp.item_base = (uint32_t*)ditems.p;
-    dp.page_present = (uint32_t*)dpresent.p;
-    dp.idx = (uint32_t*)didx.p;
+    dp.pages = (ParquetPage*)dpages;
+    dp.status = (unsigned long long*)(base + zero_at);
+    dp.item_base = (uint32_t*)(dp.status + 1 + n_proj);
+    dp.page_present = dp.item_base + items;
+    dp.idx = (uint32_t*)(base + idx_at);
     for (int q = 0; q < n_proj; q++) {
         dp.out[q].data = frame[q].data;
         dp.out[q].valid = (uint32_t*)frame[q].valid;
@@ -423,7 +493,7 @@ int parquet_scan_filter(const uint8_t* file, int64_t n, const int32_t* projectio
         const Chunk& a = plan.chunks[c0];
         const Chunk& b = plan.chunks[c1 - 1];
         if (b.unpack_end > a.unpack_begin &&
-            check_cuda(launch_snappy_decompress((const SnappyJob*)djobs.p + a.unpack_begin, b.unpack_end - a.unpack_begin,
+            check_cuda(launch_snappy_decompress((const SnappyJob*)djobs + a.unpack_begin, b.unpack_end - a.unpack_begin,
                                                 dp.status, st),
                        "Snappy decompression"))
             return kCudaError;
@@ -443,43 +513,18 @@ int parquet_scan_filter(const uint8_t* file, int64_t n, const int32_t* projectio
         if (dict && check_cuda(launch_parquet_dict_indices(dp, st), "Parquet dictionary indices")) return kCudaError;
         return check_cuda(launch_parquet_values(dp, st), "Parquet page values");
     };
-    // the copy lane starts after this stream's work so far; on every exit this stream waits for
-    // the lane before any buffer is freed
-    if (int e = check_cuda(cudaEventRecord(lane->ready, st), "cudaEventRecord")) return e;
-    if (int e = check_cuda(cudaStreamWaitEvent(lane->s, lane->ready, 0), "cudaStreamWaitEvent")) return e;
-    LaneJoin join{lane, st};
     if (direct) {
         if (!plan.chunks.empty())
             if (int e = decode(0, plan.chunks.size())) return e;
-    }
-    // Otherwise the chunks go in batches of about kBatchBytes: a batch's chunks are copied on the
-    // copy lane's stream while the batch before it is decoded on this one.
-    const int64_t kBatchBytes = batch_bytes();
-    size_t batch = 0;
-    for (size_t c0 = direct ? plan.chunks.size() : 0; c0 < plan.chunks.size(); batch++) {
-        size_t c1 = c0;
-        int64_t bytes = 0;
-        while (c1 < plan.chunks.size() && (c1 == c0 || bytes < kBatchBytes)) {
-            const Chunk& c = plan.chunks[c1];
-            if (c.bytes > 0 && check_cuda(cudaMemcpyAsync((char*)dfile.p + c.dev_off, file + c.file_off, (size_t)c.bytes,
-                                                          cudaMemcpyHostToDevice, lane->s),
-                                          "cudaMemcpyAsync"))
-                return kCudaError;
-            bytes += c.bytes;
-            c1++;
-        }
-        cudaEvent_t copied = nullptr;
-        if (int e = lane_event(*lane, batch, &copied)) return e;
-        if (int e = check_cuda(cudaEventRecord(copied, lane->s), "cudaEventRecord")) return e;
-        if (int e = check_cuda(cudaStreamWaitEvent(st, copied, 0), "cudaStreamWaitEvent")) return e;
-        if (int e = decode(c0, c1)) return e;
-        c0 = c1;
+    } else if (int e = decode_copied(file, plan, base + file_at0, st, decode)) {
+        return e;
     }
     std::vector<unsigned long long> status(1 + n_proj, 0);
-    if (int e = check_cuda(cudaMemcpyAsync(status.data(), dstatus.p, status.size() * 8, cudaMemcpyDeviceToHost, st),
+    if (int e = check_cuda(cudaMemcpyAsync(status.data(), dp.status, status.size() * 8, cudaMemcpyDeviceToHost, st),
                            "cudaMemcpyAsync"))
         return e;
     if (int e = check_cuda(cudaStreamSynchronize(st), "Parquet page decode")) return e;
+    drain.on = false;
     if (status[0])
         return set_error(kUnsupported, std::to_string(status[0]) + " malformed pages (compressed data, levels, "
                                        "dictionary indices or values that do not decode within their page)");

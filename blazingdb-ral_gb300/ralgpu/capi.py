@@ -456,7 +456,7 @@ def parquet_scan_filter(file: bytes, projections, filter_query_part: Optional[st
                         page_locked: bool = False) -> List[Column]:
     """BindableTableScan over a Parquet file (host bytes; projections = leaf indices) followed by
     its LogicalFilter (None: the scan alone).  page_locked=True hands the library the file in
-    page-locked memory, which its kernels read in place instead of copying the pages in."""
+    page-locked memory, which its kernels read in place on every system."""
     rows, dts = parquet_schema(file)
     for c in projections:
         if 0 <= c < len(dts) and dts[c] == D.GDF_invalid:

@@ -276,9 +276,10 @@ int ral_text_scan_filter_host(const char *text, int64_t n_bytes, char delimiter,
 /*
  * The same fusion over a Parquet file — a BindableTableScan of a Parquet table (parquet_parser::parse,
  * src/io/data_parser/ParquetParser.cpp:36-90, cudf's Parquet reader) followed by its LogicalFilter.
- * `file` holds the whole file (n_bytes) in host memory.  In page-locked memory the decode kernels read
- * the projected pages in place over the host link; otherwise the projected leaves' column chunks
- * are copied in, in batches decoded while the next batch is copied.  Snappy pages are decompressed
+ * `file` holds the whole file (n_bytes) in host memory.  In page-locked memory, and in any host memory
+ * where the device reads the host's pages, the decode kernels read the projected pages in place over the
+ * host link; otherwise the projected leaves' column chunks are copied in, in batches decoded while the
+ * next batch is copied.  Snappy pages are decompressed
  * on the device (one warp per page), a levels kernel decodes the definition levels of optional
  * leaves, a dictionary kernel the indices of dictionary-encoded pages, a values kernel every page's
  * values in 8192-row items, and the fused filter kernel filters the decoded columns.
