@@ -1039,24 +1039,28 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const __grid_consta
 // A dictionary-encoded page: after the bit width byte, the present rows' indices in
 // the RLE / bit-packed hybrid (a run header varint h: h odd -> (h >> 1) groups of 8 values of the
 // bit width, packed from the low bits; h even -> h >> 1 repeats of the next ceil(width / 8) bytes).
-// Thread 0 walks the run headers into a batch of segments (an RLE run, or up to kDictStage bytes of
-// a bit-packed run: a long run is cut at group boundaries), the block copies the batch's span of
-// packed bytes into shared memory with 16-byte loads, then writes the batch's indices from there,
-// each checked against the dictionary's size.  Several blocks share a page's batches.
+// A batch is a window of the stream: the block copies it into shared memory with 16-byte loads, thread 0
+// walks the run headers in it into segments (an RLE run, or the groups of a bit-packed run that lie in
+// the window), then the block writes the batch's indices from there, each checked against the
+// dictionary's size.  Several blocks share a page's batches; a window inside one long run has no header,
+// and only the block that writes its indices reads it.  Bound: the walk where runs are short, one chain of
+// dependent instructions, in 32 bits and with a header's bytes read together (700,001 rows of three
+// columns, the whole scan, against a walk byte by byte in global memory: runs of 504 values 325 -> 245 us, runs
+// of 1 to 320 values 759 -> 501 us, one run a page 132 -> 125 us).
 
 constexpr int kDictStage = 32768;  // packed index bytes staged per batch
 constexpr int kDictThreads = 1024;
-// Blocks of a page: each walks the run headers, block y decodes batches y, y + kDictSlices, ... (24 pages of
+// Blocks of a page: each walks the run headers, block y writes batches y, y + kDictSlices, ... (24 pages of
 // 131,072 indices of 6 to 12 bits, 3 to 6 batches each: 50 us with one block a page, 20 with eight).
 constexpr int kDictSlices = 8;
 
 __global__ void __launch_bounds__(kDictThreads) parquet_dict_index_kernel(const __grid_constant__ ParquetDecodeParams P) {
     __shared__ __align__(16) uint8_t s_buf[kDictStage + 64];
     __shared__ int s_row[kPqRuns + 1];
-    __shared__ long long s_info[kPqRuns];  // bit-packed: stream offset of the segment's first value; RLE: the value
+    __shared__ ral_u32 s_info[kPqRuns];  // bit-packed: the segment's first byte in s_buf; RLE: the value
     __shared__ unsigned char s_kind[kPqRuns];
     __shared__ int s_n, s_bad, s_done;
-    __shared__ long long s_pos, s_rem_groups, s_rem_pos, s_span0, s_span1;
+    __shared__ long long s_pos, s_rem;  // the stream offset reached, and the groups left of the run it is in
     const int p = P.page_lo + (int)blockIdx.x;
     const ParquetPage pg = P.pages[p];
     if (pg.dict_count <= 0 || pg.rows <= 0) return;
@@ -1074,120 +1078,108 @@ __global__ void __launch_bounds__(kDictThreads) parquet_dict_index_kernel(const 
     const uint8_t* const st = sv + 1;
     const long long nb = sbytes - 1;
     const unsigned long long mask = bw == 32 ? 0xffffffffull : ((1ull << bw) - 1ull);
-    // groups of one bit-packed segment: a batch's span stays within the stage
-    const long long seg_groups = bw > 0 ? (long long)(kDictStage - 32) / bw : (1ll << 40);
     if (threadIdx.x == 0) {
         s_pos = 0;
         s_row[0] = 0;
         s_bad = 0;
         s_done = 0;
-        s_rem_groups = 0;
-        s_rem_pos = 0;
+        s_rem = 0;
     }
     __syncthreads();
     bool out_of_range = false;
     for (int batch = 0;; ++batch) {
+        const bool mine = batch % kDictSlices == (int)blockIdx.y;
+        // the window: stream bytes [w0, w1), staged from the aligned address at or before them (inside the
+        // page's buffer, which is 16-byte padded)
+        const long long w0 = s_pos, w1 = min(w0 + kDictStage - 32, nb);
+        const uintptr_t a0 = (uintptr_t)(st + w0) & ~(uintptr_t)15;
+        const long long sbase = (long long)(a0 - (uintptr_t)st);  // stream offset of s_buf[0] (may be negative)
+        if (mine || s_rem * bw <= w1 - w0) {
+            const int nv = (int)(((uintptr_t)(st + w1) + 15 - a0) >> 4);
+            for (int i = threadIdx.x; i < nv; i += blockDim.x)
+                reinterpret_cast<uint4*>(s_buf)[i] = reinterpret_cast<const uint4*>(a0)[i];
+        }
+        __syncthreads();
         if (threadIdx.x == 0) {
-            int k = 0;
-            int row = s_row[0];
-            long long pos = s_pos, rem = s_rem_groups, rpos = s_rem_pos;
-            long long span0 = -1, span1 = -1;
+            // positions are offsets in s_buf
+            const int at0 = (int)(w0 - sbase), end = (int)(w1 - sbase);
+            const long long end_nb = nb - sbase;
+            int k = 0, row = s_row[0], pos = at0;
+            long long rem = s_rem;
             while (k < kPqRuns && row < n_idx) {
                 if (rem > 0) {
-                    // the next segment of the bit-packed run in progress
-                    if (span0 < 0) span0 = rpos;
-                    const long long room = (long long)(kDictStage - 32) - (rpos - span0);
-                    long long g = bw > 0 ? min(rem, room / bw) : rem;
-                    g = min(g, seg_groups);
-                    if (g <= 0) break;  // the stage is full: the next batch goes on from here
-                    const long long len = min(g * 8, (long long)(n_idx - row));
+                    // the groups of the bit-packed run in progress that lie in the window
+                    const long long g = rem * bw <= end - pos ? rem : (end - pos) / bw;
+                    if (g <= 0) break;
                     s_kind[k] = 1;
-                    s_info[k] = rpos;
-                    s_row[k] = row;
-                    row += (int)len;
-                    ++k;
-                    s_row[k] = row;
-                    rpos += g * bw;
-                    span1 = rpos;
+                    s_info[k] = (ral_u32)pos;
+                    s_row[k++] = row;
+                    row = (int)min(row + g * 8, (long long)n_idx);
+                    pos += (int)g * bw;
                     rem -= g;
                     continue;
                 }
-                unsigned long long h = 0;
-                int shift = 0;
-                bool ok = true;
-                while (true) {
-                    if (pos >= nb || shift > 35) {
-                        ok = false;
-                        break;
+                if (pos + 10 > end && w1 < nb) break;  // a header and an RLE run's value: up to ten bytes
+                // eight bytes from here on: a header of one or two, and a value, are read from them
+                const ral_u32* const w = reinterpret_cast<const ral_u32*>(s_buf) + (pos >> 2);
+                const ral_u32 a = w[0], b = w[1], c = w[2], sh = 8u * (ral_u32)(pos & 3);
+                const unsigned long long x = (unsigned long long)__funnelshift_r(b, c, sh) << 32 | __funnelshift_r(a, b, sh);
+                unsigned long long h;
+                ral_u32 v;  // the bytes after the header
+                int hb;
+                if (!(x & 0x80)) {
+                    hb = 1;
+                    h = x & 0x7f;
+                    v = (ral_u32)(x >> 8);
+                } else if (!(x & 0x8000)) {
+                    hb = 2;
+                    h = (x & 0x7f) | (x >> 1 & 0x3f80);
+                    v = (ral_u32)(x >> 16);
+                } else {
+                    bool more = true;
+                    h = 0;
+                    for (hb = 0; hb < 6 && pos + hb < end && more; ++hb) {
+                        const unsigned long long y = s_buf[pos + hb];
+                        h |= (y & 0x7f) << (7 * hb);
+                        more = (y & 0x80) != 0;
                     }
-                    const unsigned long long b = st[pos++];
-                    h |= (b & 0x7f) << shift;
-                    shift += 7;
-                    if (!(b & 0x80)) break;
+                    v = 0;
+                    for (int j = 0; j < 4; ++j) v |= (ral_u32)s_buf[pos + hb + j] << (8 * j);
+                    if (more) hb = 1 << 20;  // no header
                 }
-                if (!ok) {
+                pos += hb;
+                const long long after = end_nb - pos;
+                if (h & 1) rem = (long long)(h >> 1);
+                if (after < 0 || ((h & 1) ? rem * bw : (long long)vbytes) > after) {
                     s_bad = 1;
                     break;
                 }
-                if (h & 1) {
-                    const long long groups = (long long)(h >> 1);
-                    if (pos + groups * bw > nb) {
-                        s_bad = 1;
-                        break;
-                    }
-                    rem = groups;
-                    rpos = pos;
-                    pos += groups * bw;
-                } else {
-                    if (pos + vbytes > nb) {
-                        s_bad = 1;
-                        break;
-                    }
-                    unsigned long long v = 0;
-                    for (int j = 0; j < vbytes; ++j) v |= (unsigned long long)st[pos + j] << (8 * j);
-                    pos += vbytes;
-                    const long long len = min((long long)(h >> 1), (long long)(n_idx - row));
-                    if (len <= 0) continue;
-                    s_kind[k] = 0;
-                    s_info[k] = (long long)(v & mask);
-                    s_row[k] = row;
-                    row += (int)len;
-                    ++k;
-                    s_row[k] = row;
-                }
+                if (h & 1) continue;
+                pos += vbytes;
+                const int len = (int)min((long long)(h >> 1), (long long)(n_idx - row));
+                if (len <= 0) continue;
+                s_kind[k] = 0;
+                s_info[k] = v & (ral_u32)mask;
+                s_row[k++] = row;
+                row += len;
             }
-            s_pos = pos;
-            s_rem_groups = row >= n_idx ? 0 : rem;
-            s_rem_pos = rpos;
+            s_pos = sbase + pos;
+            s_rem = rem;
             s_n = k;
-            s_span0 = span0;
-            s_span1 = span1;
+            s_row[k] = row;
             if (row >= n_idx) s_done = 1;
-            else if (k == 0 && !s_bad) s_bad = 1;
+            else if (pos == at0 && k == 0) s_bad = 1;
         }
         __syncthreads();
         if (s_bad) break;
         const int n = s_n, r_lo = s_row[0], r_hi = s_row[n];
-        if (batch % kDictSlices != (int)blockIdx.y) {
+        if (!mine) {
             __syncthreads();
             if (s_done) break;
             if (threadIdx.x == 0) s_row[0] = r_hi;
             __syncthreads();
             continue;
         }
-        // the batch's packed bytes [span0, span1) into the stage: 16-byte loads from the aligned
-        // address at or before them (inside the page's buffer, which is 16-byte padded)
-        const long long span0 = s_span0, span1 = s_span1;
-        long long sbase = 0;
-        if (span0 >= 0) {
-            const uintptr_t a0 = (uintptr_t)(st + span0) & ~(uintptr_t)15;
-            const uintptr_t a1 = ((uintptr_t)(st + span1) + 15) & ~(uintptr_t)15;
-            const int nv = (int)((a1 - a0) >> 4);
-            for (int i = threadIdx.x; i < nv; i += blockDim.x)
-                reinterpret_cast<uint4*>(s_buf)[i] = reinterpret_cast<const uint4*>(a0)[i];
-            sbase = (long long)(a0 - (uintptr_t)st);  // stream offset of s_buf[0] (may be negative)
-        }
-        __syncthreads();
         for (int i = r_lo + (int)threadIdx.x; i < r_hi; i += kDictThreads) {
             int a = 0, b = n - 1;  // the last segment starting at or before i
             while (a < b) {
@@ -1197,15 +1189,15 @@ __global__ void __launch_bounds__(kDictThreads) parquet_dict_index_kernel(const 
             }
             ral_u32 v;
             if (s_kind[a]) {
-                const long long bo = (long long)(i - s_row[a]) * bw;
-                const int q = (int)(s_info[a] + (bo >> 3) - sbase);  // in the stage
+                const int bo = (i - s_row[a]) * bw;
+                const int q = (int)s_info[a] + (bo >> 3);
                 const ral_u32* const w = reinterpret_cast<const ral_u32*>(s_buf) + (q >> 2);
                 // up to 32 bits from bit sh of three words
-                const int sh = 8 * (q & 3) + (int)(bo & 7);  // below 32
+                const int sh = 8 * (q & 3) + (bo & 7);  // below 32
                 const unsigned long long x = (unsigned long long)w[1] << 32 | w[0];
                 v = (ral_u32)(x >> sh) & (ral_u32)mask;
             } else {
-                v = (ral_u32)s_info[a];
+                v = s_info[a];
             }
             if (v >= (ral_u32)pg.dict_count) {
                 out_of_range = true;
