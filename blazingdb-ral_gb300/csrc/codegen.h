@@ -99,8 +99,10 @@ struct GeneratedKernel {
     // integer-pipe double operations (softfp.cuh) unless RAL_SOFT_FP=0.  Batched item functions
     // take it from their shape (the autotuner's choice; by default the FP64 instructions, since
     // under the items' register cap the larger integer-pipe code spills: 256 programs over tables
-    // capped at 1M rows ran 31.6 ms with it against 20.4 ms without).
+    // capped at 1M rows run 9.8 ms with it against 6.4 ms without).
     bool soft_fp = true;
+    // item functions: sin / cos, double and 64-bit division are the dispatch kernel's functions
+    bool shared_ops = false;
     // relocatable item functions: register cap (0: RAL_BATCH_MAXRREG's)
     int max_registers = 0;
     // dynamic shared memory a block needs (staged eval kernels)

@@ -32,7 +32,9 @@ typedef unsigned int ral_u32;
 #if RAL_SOFT_FP
 RAL_FI ral_i64 ral_d2i(double d) { return ral_sf_d2i(d); }
 RAL_FI double ral_i2d(ral_i64 x) { return ral_sf_i2d(x); }
+#ifndef RAL_SHARED_OPS
 RAL_FI double ral_ddiv(double a, double b) { return ral_sf_div(a, b); }
+#endif
 // RAL_SOFT_ROUND 0: floor / ceil by the FP64 pipe's rounding instruction (one FP64 instruction
 // against ~28 integer ones; same bits), the other operations staying on the integer pipes
 #ifndef RAL_SOFT_ROUND
@@ -56,7 +58,9 @@ RAL_FI float ral_d2f(double d) { return ral_sf_d2f(d); }
 #else
 RAL_FI ral_i64 ral_d2i(double d) { return __double2ll_rz(d); }
 RAL_FI double ral_i2d(ral_i64 x) { return __ll2double_rn(x); }
+#ifndef RAL_SHARED_OPS
 RAL_FI double ral_ddiv(double a, double b) { return __ddiv_rn(a, b); }
+#endif
 RAL_FI double ral_dfloor(double x) { return floor(x); }
 RAL_FI double ral_dceil(double x) { return ceil(x); }
 RAL_FI bool ral_dlt(double a, double b) { return a < b; }
@@ -68,16 +72,24 @@ RAL_FI bool ral_dne(double a, double b) { return a != b; }
 RAL_FI double ral_f2d(float f) { return (double)f; }
 RAL_FI float ral_d2f(double d) { return __double2float_rn(d); }
 #endif
-// sin / cos: RAL_SOFT_TRIG 0 (the default) uses the library functions, 1 the integer-pipe
-// versions of softfp.cuh (within one ulp).  Unlike the exact operations above the two differ in
-// the last bit, so the choice is the same for every kernel of a process.  Measured on GB300 the
-// library functions are faster: the 256-program mix ran 138 ms batched / 158 ms as plain calls
-// with them and 155 / 172 ms with the integer-pipe versions (whose two polynomial paths diverge
-// within a warp by quadrant).
+// sin / cos: RAL_SOFT_TRIG 1 (the default) uses the integer-pipe versions of softfp.cuh, 0 the library
+// functions.  Unlike the exact operations above the two differ in the last bit, so the choice is the
+// same for every kernel of a process.
 #ifndef RAL_SOFT_TRIG
-#define RAL_SOFT_TRIG 0
+#define RAL_SOFT_TRIG 1
 #endif
-#if RAL_SOFT_TRIG
+// Item functions call these (they are the dispatch kernel's; bits as below and above)
+#if defined(RAL_SHARED_OPS)
+extern "C" __device__ double ral_shared_ddiv(double a, double b);
+extern "C" __device__ ral_i64 ral_shared_divi(ral_i64 a, ral_i64 b);
+extern "C" __device__ ral_i64 ral_shared_modi(ral_i64 a, ral_i64 b);
+RAL_FI double ral_ddiv(double a, double b) { return ral_shared_ddiv(a, b); }
+#endif
+#if RAL_SOFT_TRIG && defined(RAL_SHARED_OPS)
+extern "C" __device__ double ral_shared_trig(double x, int want_cos);
+RAL_FI double ral_dsin(double x) { return ral_shared_trig(x, 0); }
+RAL_FI double ral_dcos(double x) { return ral_shared_trig(x, 1); }
+#elif RAL_SOFT_TRIG
 RAL_FI double ral_dsin(double x) { return ral_sf_sin(x); }
 RAL_FI double ral_dcos(double x) { return ral_sf_cos(x); }
 #else
@@ -119,7 +131,8 @@ RAL_FI ral_i64 ral_muli(ral_i64 a, ral_i64 b) { return (ral_i64)((ral_u64)a * (r
 // bits; 1 uses the integer-only division for every divisor.  All are exact.  Measured on the
 // 12-op projection (200M rows, divisors in [1, 1000]): 3 = 3.32 ms, 0 = 3.78 ms, 2 = 3.97 ms,
 // 1 = 4.6 ms -- the 2-by-1 and Newton versions free the FP64 pipe but cost more integer work
-// than they save there; the word steps cost little of either.
+// than they save there; the word steps cost little of either.  Item functions always divide by the
+// integer-only division, in one place for all of them.
 #ifndef RAL_SOFT_INT_DIV
 #define RAL_SOFT_INT_DIV 3
 #endif
@@ -131,6 +144,10 @@ RAL_FI bool ral_tiny_divisor(ral_i64 b) {
     const ral_u64 m = b < 0 ? 0ull - (ral_u64)b : (ral_u64)b;
     return m < 0x10000ull;
 }
+#if defined(RAL_SHARED_OPS)
+RAL_FI ral_i64 ral_divi(ral_i64 a, ral_i64 b) { return ral_shared_divi(a, b); }
+RAL_FI ral_i64 ral_modi(ral_i64 a, ral_i64 b) { return ral_shared_modi(a, b); }
+#else
 RAL_FI ral_i64 ral_divi(ral_i64 a, ral_i64 b) {
     if (b == 0) return 0;
     if (b == -1) return (ral_i64)(0ull - (ral_u64)a);
@@ -156,6 +173,7 @@ RAL_FI ral_i64 ral_modi(ral_i64 a, ral_i64 b) {
     return a % b;
 #endif
 }
+#endif
 // ral_divi / ral_modi for kernels that keep the reciprocals m(d) = floor((2^32 - 1) / d) of the
 // divisors below RAL_RCP_TAB in a shared-memory table (the eval kernel of a program that divides
 // by a column): m is the table's entry for |b|, or 0 when |b| is not below RAL_RCP_TAB (then the

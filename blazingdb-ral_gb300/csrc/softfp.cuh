@@ -668,21 +668,31 @@ RAL_SF long long ral_sf_modc(long long n, long long d, long long mult, long long
 
 // ---- sine and cosine ---------------------------------------------------------------------------
 
-// 64-bit value V (a leading one anywhere) times 2^E, rounded to nearest even as a double (normal
-// results only; the callers' values lie in [2^-30, 2])
+RAL_SF unsigned int ral_sf_funnel_r(unsigned int lo, unsigned int hi, unsigned int n) {  // n < 32
+#if defined(__CUDA_ARCH__)
+    return __funnelshift_r(lo, hi, n);
+#else
+    return (unsigned int)(((unsigned long long)hi << 32 | lo) >> n);
+#endif
+}
+
+// 64-bit value V >= 2^32 times 2^E, rounded to nearest as a double (normal results only)
 RAL_SF double ral_sf_pack(unsigned long long V, int E, unsigned long long sign) {
-    const int lz = ral_sf_clz64(V);
+#if defined(__CUDA_ARCH__)
+    const int lz = __clz((int)(V >> 32));
+#else
+    const int lz = __builtin_clz((unsigned)(V >> 32));
+#endif
     V <<= lz;
-    E -= lz;
-    unsigned long long m = V >> 11;
-    const unsigned long long rest = V & 0x7ffull;
-    if (rest > 0x400ull || (rest == 0x400ull && (m & 1u))) m += 1;
-    int be = E + 63 + 1023;
-    if (m == (1ull << 53)) {
-        m >>= 1;
-        be += 1;
-    }
-    return ral_sf_double(sign | ((unsigned long long)be << 52) | (m & RAL_SF_FRAC));
+    // the significand in [2^52, 2^53], whose leading one counts in the exponent field
+    const unsigned long long m = (V >> 11) + ((V >> 10) & 1ull);
+    return ral_sf_double((sign | ((unsigned long long)(unsigned)(E - lz + 63 + 1022) << 52)) + m);
+}
+
+// the high word of a * b, or one or two less (the product of the low halves left out)
+RAL_SF unsigned long long ral_sf_umulh_near(unsigned long long a, unsigned long long b) {
+    const unsigned a0 = (unsigned)a, a1 = (unsigned)(a >> 32), b0 = (unsigned)b, b1 = (unsigned)(b >> 32);
+    return (unsigned long long)a1 * b1 + ral_sf_umulhi32(a1, b0) + ral_sf_umulhi32(a0, b1);
 }
 
 // Fixed-point constants, each the nearest (or, for 2/pi and pi/2, the truncated) value:
@@ -693,121 +703,156 @@ RAL_SF double ral_sf_pack(unsigned long long V, int E, unsigned long long sign) 
 #define RAL_SF_2PI_W0 0xdb6295993c439041ull
 #define RAL_SF_PI2_HI 0xc90fdaa22168c234ull
 #define RAL_SF_PI2_LO 0xc4c6628b80dc1cd1ull
-
-// sin(|r|) (want_cos false) or cos(|r|) for r = rm * 2^-(64 + sr), rm normalised, |r| <= pi/4
-RAL_SF double ral_sf_sincos_poly(unsigned long long rm, int sr, bool want_cos, unsigned long long sign) {
-    const unsigned long long zz = ral_sf_umulh(rm, rm);  // r^2 * 2^(64 + 2 sr)
-    const unsigned long long z = 2 * sr >= 64 ? 0ull : (zz >> (2 * sr));  // r^2 in Q0.64
-    if (want_cos) {
-        // 2^63 / (2n)!, n = 10 .. 0
-        const unsigned long long c[11] = {0x8000000000000000ull, 0x4000000000000000ull, 0x0555555555555555ull,
-                                          0x002d82d82d82d82eull, 0x0000d00d00d00d01ull, 0x0000024fc9f6ef14ull,
-                                          0x000000047bb63bfeull, 0x00000000064e5d2aull, 0x000000000006b9fdull,
-                                          0x00000000000005a1ull, 0x0000000000000004ull};
-        unsigned long long p = c[10];
-#pragma unroll
-        for (int n = 9; n >= 0; --n) p = c[n] - ral_sf_umulh(p, z);
-        return ral_sf_pack(p, -63, sign);
-    }
-    // 2^63 / (2n+1)!, n = 9 .. 0
+RAL_SF unsigned long long ral_sf_cos_coef(int n) {
+    const unsigned long long c[11] = {0x8000000000000000ull, 0x4000000000000000ull, 0x0555555555555555ull,
+                                      0x002d82d82d82d82eull, 0x0000d00d00d00d01ull, 0x0000024fc9f6ef14ull,
+                                      0x000000047bb63bfeull, 0x00000000064e5d2aull, 0x000000000006b9fdull,
+                                      0x00000000000005a1ull, 0x0000000000000004ull};
+    return c[n];
+}
+RAL_SF unsigned long long ral_sf_sin_coef(int n) {
     const unsigned long long c[10] = {0x8000000000000000ull, 0x1555555555555555ull, 0x0111111111111111ull,
                                       0x0006806806806807ull, 0x0000171de3a556c7ull, 0x00000035cc8acfebull,
                                       0x000000005849184full, 0x00000000006b9fd0ull, 0x000000000000654bull,
                                       0x000000000000004cull};
-    unsigned long long p = c[9];
-#pragma unroll
-    for (int n = 8; n >= 0; --n) p = c[n] - ral_sf_umulh(p, z);
-    // sin(r) = r * p: value = umulh(rm, p) * 2^(-63 - sr)
-    return ral_sf_pack(ral_sf_umulh(rm, p), -63 - sr, sign);
+    return c[n];
 }
 
-RAL_SF double ral_sf_hw_sin(double x) {
-#if defined(__CUDA_ARCH__)
-    return sin(x);
-#else
-    return __builtin_sin(x);
-#endif
+// sin(r) (use_cos false) or cos(r) for r = rm * 2^-(63 + L) <= pi/4, rm >= 2^62, L >= 1.  One Horner chain for
+// both, its coefficients selected, so that the lanes of a warp stay together; the terms below 2^-28 of
+// the result in 32 bits (their truncation and that of the products: below 2^-60 of the result).
+RAL_SF double ral_sf_sincos_poly(unsigned long long rm, int L, bool use_cos, unsigned long long sign) {
+    const int down = 2 * L - 2;  // r^2 in Q0.64 is rm^2 / 2^64 shifted down by this
+    const unsigned long long z = down < 64 ? ral_sf_umulh_near(rm, rm) >> down : 0ull;
+    const unsigned zh = (unsigned)(z >> 32);
+#define RAL_SF_COEF(n) (use_cos ? ral_sf_cos_coef(n) : ral_sf_sin_coef(n))
+    unsigned t = (unsigned)RAL_SF_COEF(9);
+    t = (unsigned)RAL_SF_COEF(8) - ral_sf_umulhi32(t, zh);
+    t = (unsigned)RAL_SF_COEF(7) - ral_sf_umulhi32(t, zh);
+    unsigned long long p = RAL_SF_COEF(6) - ral_sf_umulhi32(t, zh);
+    p = RAL_SF_COEF(5) - ((p >> 32) * zh + ral_sf_umulhi32((unsigned)p, zh));
+    p = RAL_SF_COEF(4) - ral_sf_umulh_near(p, z);
+    p = RAL_SF_COEF(3) - ral_sf_umulh_near(p, z);
+    p = RAL_SF_COEF(2) - ral_sf_umulh_near(p, z);
+    p = RAL_SF_COEF(1) - ral_sf_umulh_near(p, z);
+    p = ral_sf_cos_coef(0) - ral_sf_umulh_near(p, z);
+#undef RAL_SF_COEF
+    const unsigned long long v = ral_sf_umulh_near(rm, p);  // sin(r) = r * p
+    return ral_sf_pack(use_cos ? p : v, use_cos ? -63 : -62 - L, sign);
 }
-RAL_SF double ral_sf_hw_cos(double x) {
-#if defined(__CUDA_ARCH__)
-    return cos(x);
+
+// sin(x) = [s, c, -s, -c][q], cos(x) = [c, -s, -c, s][q] with s = sin r, c = cos r for x = q pi/2 + r and
+// r negative where rneg; all for |x|, sin's sign then following x's
+RAL_SF double ral_sf_sincos_quadrant(unsigned long long rm, int L, unsigned q, bool rneg, bool want_cos, unsigned long long xsign) {
+    const unsigned k = q + (want_cos ? 1u : 0u);
+    const bool use_cos = (k & 1u) != 0;
+    const bool neg = ((k & 2u) != 0) ^ (!use_cos && rneg) ^ (!want_cos && xsign != 0);
+    return ral_sf_sincos_poly(rm, L, use_cos, neg ? RAL_SF_SIGN : 0ull);
+}
+
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
+#define RAL_SF_CALL static __host__ __device__ __noinline__
 #else
-    return __builtin_cos(x);
+#define RAL_SF_CALL static inline
+#endif
+// The arguments that the form below leaves: 2^52 and more, infinities and NaN (the library's functions),
+// and those close to a multiple of pi/2, with 192 bits of 2/pi and 128 of the fraction.
+RAL_SF_CALL double ral_sf_sincos_far(double x, bool want_cos) {
+    const unsigned long long X = ral_sf_obits(x);
+    const int ex = (int)((X >> 52) & 0x7ff);
+    if (ex < 1075 && ex >= 1022) {
+        const unsigned long long m = (X & RAL_SF_FRAC) | RAL_SF_IMPL;
+        // P = m * (2/pi * 2^192), its upper three words: |x| * 2/pi = P * 2^-(192 + v)
+        const int v = 1075 - ex;
+        const unsigned long long p1a = ral_sf_umulh(m, RAL_SF_2PI_W0), p1 = p1a + m * RAL_SF_2PI_W1;
+        const unsigned long long p2a = ral_sf_umulh(m, RAL_SF_2PI_W1) + (p1 < p1a ? 1ull : 0ull), p2 = p2a + m * RAL_SF_2PI_W2;
+        const unsigned long long p3 = ral_sf_umulh(m, RAL_SF_2PI_W2) + (p2 < p2a ? 1ull : 0ull);
+        unsigned q = (unsigned)(p3 >> v);
+        unsigned long long fhi = (p2 >> v) | (p3 << (64 - v)), flo = (p1 >> v) | (p2 << (64 - v));
+        const bool rneg = (fhi >> 63) != 0;  // f >= 1/2: the nearer multiple is the next
+        if (rneg) {
+            q += 1u;
+            flo = 0ull - flo;
+            fhi = ~fhi + (flo == 0 ? 1ull : 0ull);
+        }
+        if ((fhi | flo) != 0) {
+            // r = f * pi/2 by the three high partial products, normalised
+            const unsigned long long ac = fhi * RAL_SF_PI2_HI;
+            unsigned long long lo = ac + ral_sf_umulh(fhi, RAL_SF_PI2_LO);
+            unsigned long long hi = ral_sf_umulh(fhi, RAL_SF_PI2_HI) + (lo < ac ? 1ull : 0ull);
+            const unsigned long long bc = ral_sf_umulh(flo, RAL_SF_PI2_HI);
+            lo += bc;
+            hi += lo < bc ? 1ull : 0ull;
+            // (f * pi/2) = hi:lo * 2^-127
+            const int lz = hi ? ral_sf_clz64(hi) : 64 + ral_sf_clz64(lo | 1ull);
+            const unsigned long long rm = hi ? (lz ? hi << lz | lo >> (64 - lz) : hi) : lo << (lz - 64);
+            if (rm >> 63) return ral_sf_sincos_quadrant(rm, lz, q, rneg, want_cos, X & RAL_SF_SIGN);
+        }
+    }
+#if defined(__CUDA_ARCH__)
+    return want_cos ? cos(x) : sin(x);
+#else
+    return want_cos ? __builtin_cos(x) : __builtin_sin(x);
 #endif
 }
 
-// sin(x) (want_cos false) or cos(x) within one ulp, for 2^-26 <= |x| < 2^20; other inputs use
-// the library functions.  Method: Payne-Hanek-style reduction x * 2/pi = k + f with a 192-bit
-// fixed-point 2/pi (exact product with the 53-bit significand), r = f * pi/2 to 128 bits, then
-// the Taylor series of sin(r)/r or cos(r) in 64-bit fixed point by Horner's rule.
+// sin(x) (want_cos false) or cos(x), within 0.51 ulp for |x| < 2^52.  Payne and Hanek's reduction in 32-bit
+// words: |x| * 2/pi = q + f from a product of 53 by 128 bits, of which 96 fraction bits are kept (arguments so
+// close to a multiple of pi/2 that these do not give f's leading 64 bits go to ral_sf_sincos_far), r = f * pi/2
+// and a series in 64-bit fixed point.
+//
+// About 200 integer instructions against some 20 FP64 ones of the library's function, each of which takes the
+// FP64 pipe as long as 64 integer instructions take the SM: a projection of SIN over 50M rows 570 us (1798
+// with the library's), of SIN(COS(SIN(x * y))) 1409 (5255), 256 programs over tables of up to 1M rows
+// 7.2 ms (16.2).
 RAL_SF double ral_sf_sincos(double x, bool want_cos) {
     const unsigned long long X = ral_sf_obits(x);
     const int ex = (int)((X >> 52) & 0x7ff);
-    const unsigned long long xsign = X & RAL_SF_SIGN;
-    if (ex < 1023 - 26 || ex >= 1023 + 20) return want_cos ? ral_sf_hw_cos(x) : ral_sf_hw_sin(x);
+    if (ex < 1023 - 27) return want_cos ? 1.0 : x;  // their own rounding
     const unsigned long long m = (X & RAL_SF_FRAC) | RAL_SF_IMPL;
-    const int e2 = ex - 1075;  // x = m * 2^e2
-    unsigned long long rm;
-    int sr;
-    unsigned q;
+    unsigned long long rm = m << 11;  // |x| < 1/2: r = |x|
+    int L = 1023 - ex;
+    unsigned q = 0;
     bool rneg = false;
-    if ((X & ~RAL_SF_SIGN) < 0x3fe921fb54442d18ull) {  // |x| < pi/4: r = x exactly
-        rm = m << 11;
-        sr = -53 - e2;
-        q = 0;
-    } else {
-        // P = m * (2/pi * 2^192), four words
-        const unsigned long long t0 = m * RAL_SF_2PI_W0, h0 = ral_sf_umulh(m, RAL_SF_2PI_W0);
-        const unsigned long long t1 = m * RAL_SF_2PI_W1, h1 = ral_sf_umulh(m, RAL_SF_2PI_W1);
-        const unsigned long long t2 = m * RAL_SF_2PI_W2, h2 = ral_sf_umulh(m, RAL_SF_2PI_W2);
-        (void)t0;
-        const unsigned long long p1 = h0 + t1;
-        const unsigned long long a1 = p1 < h0 ? 1ull : 0ull;
-        const unsigned long long s2 = h1 + t2;
-        const unsigned long long a2a = s2 < h1 ? 1ull : 0ull;
-        const unsigned long long p2 = s2 + a1;
-        const unsigned long long a2 = a2a + (p2 < s2 ? 1ull : 0ull);
-        const unsigned long long p3 = h2 + a2;
-        // x * 2/pi = P * 2^(e2 - 192): sh = 192 - e2 fraction bits, v = sh - 192 in [33, 53]
-        const int v = -e2;
-        unsigned long long k = p3 >> v;
-        unsigned long long fhi = (p2 >> v) | (p3 << (64 - v));
-        unsigned long long flo = (p1 >> v) | (p2 << (64 - v));
-        if (fhi >> 63) {  // f >= 1/2: the nearer quadrant is k + 1, and r = (f - 1) pi/2 < 0
-            k += 1;
-            flo = 0ull - flo;
-            fhi = ~fhi + (flo == 0 ? 1ull : 0ull);
-            rneg = true;
-        }
-        q = (unsigned)(k & 3u);
-        // r = f * pi/2 in Q0.128: (f * pi2) >> 127, from the three high partial products
-        const unsigned long long ac_lo = fhi * RAL_SF_PI2_HI, ac_hi = ral_sf_umulh(fhi, RAL_SF_PI2_HI);
-        const unsigned long long ad = ral_sf_umulh(fhi, RAL_SF_PI2_LO), bc = ral_sf_umulh(flo, RAL_SF_PI2_HI);
-        unsigned long long lo = ac_lo + ad;
-        unsigned long long hi = ac_hi + (lo < ac_lo ? 1ull : 0ull);
-        const unsigned long long lo2 = lo + bc;
-        hi += lo2 < lo ? 1ull : 0ull;
-        lo = lo2;
-        const unsigned long long rhi = (hi << 1) | (lo >> 63), rlo = lo << 1;
-        if (rhi != 0) {
-            const int lz = ral_sf_clz64(rhi);
-            rm = lz ? ((rhi << lz) | (rlo >> (64 - lz))) : rhi;
-            sr = lz;
-        } else {
-            if (rlo == 0) return want_cos ? ral_sf_hw_cos(x) : ral_sf_hw_sin(x);
-            const int lz = ral_sf_clz64(rlo);
-            rm = rlo << lz;
-            sr = 64 + lz;
-        }
+    if (ex >= 1022) {
+        const unsigned m0 = (unsigned)m, m1 = (unsigned)(m >> 32);
+        const unsigned c0 = (unsigned)RAL_SF_2PI_W1, c1 = (unsigned)(RAL_SF_2PI_W1 >> 32);
+        const unsigned c2 = (unsigned)RAL_SF_2PI_W2, c3 = (unsigned)(RAL_SF_2PI_W2 >> 32);
+        // w5 .. w1 of m * (2/pi * 2^128); |x| * 2/pi = w * 2^-(128 + v), v = 1075 - ex in 1 .. 53
+        unsigned long long t = (unsigned long long)m0 * c1 + ral_sf_umulhi32(m0, c0);
+        unsigned long long u = (unsigned long long)m1 * c0 + (unsigned)t;
+        const unsigned w1 = (unsigned)u;
+        t = (unsigned long long)m0 * c2 + (t >> 32);
+        u = (unsigned long long)m1 * c1 + (unsigned)t + (u >> 32);
+        const unsigned w2 = (unsigned)u;
+        t = (unsigned long long)m0 * c3 + (t >> 32);
+        u = (unsigned long long)m1 * c2 + (unsigned)t + (u >> 32);
+        const unsigned w3 = (unsigned)u;
+        u = (unsigned long long)m1 * c3 + (t >> 32) + (u >> 32);
+        const unsigned w4 = (unsigned)u, w5 = (unsigned)(u >> 32);
+        const int v = 1075 - ex;
+        const bool high = v >= 32;
+        const unsigned h = high ? 0u : w5, a = high ? w5 : w4, b = high ? w4 : w3, c = high ? w3 : w2, d = high ? w2 : w1;
+        const unsigned sh = (unsigned)v & 31u;
+        q = ral_sf_funnel_r(a, h, sh);
+        unsigned f2 = ral_sf_funnel_r(b, a, sh), f1 = ral_sf_funnel_r(c, b, sh), f0 = ral_sf_funnel_r(d, c, sh);
+        const unsigned up = (unsigned)((int)f2 >> 31);  // f >= 1/2: the nearer multiple is the next
+        q -= up;
+        rneg = up != 0u;
+        f2 ^= up;
+        f1 ^= up;
+        f0 ^= up;
+#if defined(__CUDA_ARCH__)
+        L = __clz((int)f2);
+#else
+        L = f2 ? __builtin_clz(f2) : 32;
+#endif
+        if (L > 31 || L > v + 8 || v < 1) return ral_sf_sincos_far(x, want_cos);
+        // 64 bits of f, normalised, times pi/2
+        const unsigned g1 = ral_sf_funnel_r(f1, f2, 32u - L), g0 = ral_sf_funnel_r(f0, f1, 32u - L);
+        rm = ral_sf_umulh_near((unsigned long long)g1 << 32 | g0, RAL_SF_PI2_HI);
     }
-    // quadrant: sin(x) = [s, c, -s, -c][q], cos(x) = [c, -s, -c, s][q] with s = sin r, c = cos r
-    const bool use_cos = want_cos ? (q & 1u) == 0 : (q & 1u) == 1;
-    bool neg;
-    if (want_cos) neg = (q == 1 || q == 2);
-    else neg = (q >= 2);
-    if (!use_cos && rneg) neg = !neg;               // sin(-|r|) = -sin|r|
-    if (!want_cos && xsign) neg = !neg;             // sin(-x) = -sin x; cos is even
-    return ral_sf_sincos_poly(rm, sr, use_cos, neg ? RAL_SF_SIGN : 0ull);
+    return ral_sf_sincos_quadrant(rm, L, q, rneg, want_cos, X & RAL_SF_SIGN);
 }
 
 RAL_SF double ral_sf_sin(double x) { return ral_sf_sincos(x, false); }
