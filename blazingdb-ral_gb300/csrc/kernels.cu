@@ -678,14 +678,85 @@ __device__ __forceinline__ LevelRun ral_level_run(const uint8_t* w, int at, int 
     return r;
 }
 
+constexpr int kLevelThreads = 1024;
+
+// Rows [rel0, rel1) of a required page of PLAIN values, by 256 threads of which this one is t.
+__device__ __forceinline__ void ral_pq_plain_rows(const ParquetPage& pg, const ParquetColumnOut& col, int rel0, int rel1, int t) {
+    const int lane = t & 31, warp = t >> 5, w = col.width;
+    const uint8_t* const vals = (const uint8_t*)pg.data + pg.values_off;
+    // Every row has its value (the page's length is checked on the host).  The lanes of a
+    // warp take consecutive rows: each loads the aligned word where its value starts and
+    // takes the next word from the lane after it (the last lane of the run loads it), so a
+    // warp reads one contiguous aligned span whatever the values' alignment.
+    const uintptr_t va = (uintptr_t)vals;
+    if (w == 8) {
+        // 16-byte words: lane l takes rows 2m, 2m + 1 (m = the warp's pair + l), bytes
+        // [s + 16m, s + 16m + 16) past the aligned base: word m and, when s > 0, word m + 1
+        // from the next lane (the last lane of the run loads it, when its values reach it)
+        const int s16 = (int)(va & 15);
+        const int k = s16 >> 2, f = (s16 & 3) * 8;
+        const uint4* q = reinterpret_cast<const uint4*>(va - s16);
+        unsigned long long* out = reinterpret_cast<unsigned long long*>(col.data) + pg.row_start;
+#pragma unroll 2
+        for (int m0 = (rel0 >> 1) + 32 * warp; 2 * m0 < rel1; m0 += 256) {
+            const int m = m0 + lane;
+            const int r = 2 * m;
+            const bool in = r < rel1;
+            const uint4 a = in ? q[m] : make_uint4(0u, 0u, 0u, 0u);
+            uint4 b;
+            b.x = __shfl_down_sync(0xffffffffu, a.x, 1);
+            b.y = __shfl_down_sync(0xffffffffu, a.y, 1);
+            b.z = __shfl_down_sync(0xffffffffu, a.z, 1);
+            b.w = __shfl_down_sync(0xffffffffu, a.w, 1);
+            const bool two = r + 1 < rel1;
+            if (in && (lane == 31 || r + 2 >= rel1) && s16 + (two ? 16 : 8) > 16) b = q[m + 1];
+            ral_u32 o0, o1, o2, o3;
+            switch (k) {  // uniform over the page
+            case 0: o0 = a.x; o1 = a.y; o2 = a.z; o3 = a.w; if (f) { o0 = __funnelshift_r(a.x, a.y, f); o1 = __funnelshift_r(a.y, a.z, f); o2 = __funnelshift_r(a.z, a.w, f); o3 = __funnelshift_r(a.w, b.x, f); } break;
+            case 1: o0 = __funnelshift_r(a.y, a.z, f); o1 = __funnelshift_r(a.z, a.w, f); o2 = __funnelshift_r(a.w, b.x, f); o3 = __funnelshift_r(b.x, b.y, f); break;
+            case 2: o0 = __funnelshift_r(a.z, a.w, f); o1 = __funnelshift_r(a.w, b.x, f); o2 = __funnelshift_r(b.x, b.y, f); o3 = __funnelshift_r(b.y, b.z, f); break;
+            default: o0 = __funnelshift_r(a.w, b.x, f); o1 = __funnelshift_r(b.x, b.y, f); o2 = __funnelshift_r(b.y, b.z, f); o3 = __funnelshift_r(b.z, b.w, f); break;
+            }
+            if (in) out[r] = (unsigned long long)o1 << 32 | o0;
+            if (two) out[r + 1] = (unsigned long long)o3 << 32 | o2;
+        }
+    } else {
+        const int sh = (int)(va & 3) * 8;
+        const ral_u32* q = reinterpret_cast<const ral_u32*>(va - (va & 3));
+        ral_u32* out = reinterpret_cast<ral_u32*>(col.data) + pg.row_start;
+#pragma unroll 4
+        for (int r0 = rel0 + 32 * warp; r0 < rel1; r0 += 256) {
+            const int r = r0 + lane;
+            const bool in = r < rel1;
+            const ral_u32 lo = in ? q[r] : 0u;
+            ral_u32 nx = __shfl_down_sync(0xffffffffu, lo, 1);
+            if (sh && in && (lane == 31 || r + 1 >= rel1)) nx = q[r + 1];
+            if (in) out[r] = sh ? (lo >> sh) | (nx << (32 - sh)) : lo;
+        }
+    }
+}
+
+// The page of an item: the last one whose first item is at or before it.
+__device__ __forceinline__ int ral_pq_page_of(const ParquetDecodeParams& P, int item) {
+    int a = P.page_lo, b = P.page_hi - 1;
+    while (a < b) {
+        const int m = (a + b + 1) >> 1;
+        if (P.pages[m].item0 <= item) a = m;
+        else b = m - 1;
+    }
+    return a;
+}
+
 // One block per optional page.  The run headers form a chain of which only the start is known.  Every
 // byte of a 12 KiB window of the stream is read as if a header started there, by all threads, which
 // leaves the bytes to the next one; thread 0 then only adds hops (some 45 cycles a run), and the runs it
 // lists are read a thread each into a table, from which every thread writes 32 rows' validity at a time.
 // Bound: the latency of a page's steps (one block a page).  24 pages of 131,072 rows, 12 of them with 3%
-// nulls (15.6 KB, 600 runs): 73 us, against 141 us when thread 0 read every header itself.  (Composing the
-// hops of 32-byte segments in parallel and writing bits a run a thread measured 205 us.)
-__global__ void __launch_bounds__(256) parquet_levels_kernel(const __grid_constant__ ParquetDecodeParams P) {
+// nulls (15.6 KB, 600 runs): 46 us, 72 with 256 threads a block and 141 when thread 0 read every header
+// itself.  (Composing the hops of 32-byte segments in parallel and writing bits a run a thread measured
+// 205 us.)  These few blocks leave the device and the link to the file idle: further blocks write the values
+// of required PLAIN pages, which wait for nothing (the scan with these pages 198 -> 183 us).
+__global__ void __launch_bounds__(kLevelThreads) parquet_levels_kernel(const __grid_constant__ ParquetDecodeParams P) {
     __shared__ ral_u32 s_lw[kPqWindow / 4 + 8];
     __shared__ uint16_t s_hop[kPqWindow];  // per byte of the window: the bytes to the next header if one starts there
     __shared__ uint16_t s_start[kPqRuns];
@@ -693,7 +764,16 @@ __global__ void __launch_bounds__(256) parquet_levels_kernel(const __grid_consta
     __shared__ int s_info[kPqRuns];  // bit-packed: byte offset of the run's levels; RLE: the level
     __shared__ unsigned char s_kind[kPqRuns];
     __shared__ int s_n, s_new, s_bad, s_emit, s_emit_end, s_done;
-    __shared__ long long s_pos, s_w[8];
+    __shared__ long long s_pos, s_w[kLevelThreads / 32];
+    if ((int)blockIdx.x >= P.page_hi - P.page_lo) {
+        const int item = P.item_lo + ((int)blockIdx.x - (P.page_hi - P.page_lo)) * (kLevelThreads / 256) + (int)(threadIdx.x >> 8);
+        if (item >= P.item_hi) return;
+        const ParquetPage pg = P.pages[ral_pq_page_of(P, item)];
+        if (pg.optional || pg.dict_count > 0) return;
+        const int rel0 = (item - pg.item0) * kParquetItemRows;
+        ral_pq_plain_rows(pg, P.out[pg.column], rel0, min(rel0 + kParquetItemRows, pg.rows), threadIdx.x & 255);
+        return;
+    }
     const ParquetPage pg = P.pages[P.page_lo + blockIdx.x];
     if (!pg.optional || pg.rows <= 0) return;
     const ParquetColumnOut col = P.out[pg.column];
@@ -723,10 +803,10 @@ __global__ void __launch_bounds__(256) parquet_levels_kernel(const __grid_consta
             w0 = pos;
             off = (int)((uintptr_t)(lev + w0) & 3);
             have = min(kPqWindow + 16, lev_bytes - w0);
-            for (int i = threadIdx.x; i < (off + have + 3) >> 2; i += 256)
+            for (int i = threadIdx.x; i < (off + have + 3) >> 2; i += kLevelThreads)
                 s_lw[i] = reinterpret_cast<const ral_u32*>(lev + w0 - off)[i];
             __syncthreads();
-            for (int p = threadIdx.x; p < min(kPqWindow, have); p += 256)
+            for (int p = threadIdx.x; p < min(kPqWindow, have); p += kLevelThreads)
                 s_hop[p] = (uint16_t)min(ral_level_run(reinterpret_cast<const uint8_t*>(s_lw) + off, p, lev_bytes - w0).hop, 0xffff);
             __syncthreads();
         }
@@ -744,11 +824,11 @@ __global__ void __launch_bounds__(256) parquet_levels_kernel(const __grid_consta
         }
         __syncthreads();
         const int fresh = s_new;
-        LevelRun run[kPqRuns / 256];
+        LevelRun run[kPqRuns / kLevelThreads];
         long long rows = 0;  // this thread's runs' rows, and (above 2^40) how many of them have some
 #pragma unroll
-        for (int q = 0; q < kPqRuns / 256; ++q) {
-            const int k = (int)threadIdx.x * (kPqRuns / 256) + q;
+        for (int q = 0; q < kPqRuns / kLevelThreads; ++q) {
+            const int k = (int)threadIdx.x * (kPqRuns / kLevelThreads) + q;
             run[q].len = 0;
             if (k < fresh) {
                 run[q] = ral_level_run(sb, s_start[k], lev_bytes - w0);
@@ -765,7 +845,7 @@ __global__ void __launch_bounds__(256) parquet_levels_kernel(const __grid_consta
         if (lane == 31) s_w[warp] = inc;
         __syncthreads();
         long long before = inc - rows, total = 0;
-        for (int w = 0; w < 8; ++w) {
+        for (int w = 0; w < kLevelThreads / 32; ++w) {
             if (w < warp) before += s_w[w];
             total += s_w[w];
         }
@@ -773,7 +853,7 @@ __global__ void __launch_bounds__(256) parquet_levels_kernel(const __grid_consta
         int slot = carried + (int)(before >> 44);
         __syncthreads();
 #pragma unroll
-        for (int q = 0; q < kPqRuns / 256; ++q) {
+        for (int q = 0; q < kPqRuns / kLevelThreads; ++q) {
             if (run[q].len <= 0) continue;  // runs of no rows are left out
             s_kind[slot] = run[q].packed ? 1 : 0;
             s_info[slot] = run[q].packed ? w0 + run[q].pay : sb[run[q].pay] & 1;
@@ -792,7 +872,7 @@ __global__ void __launch_bounds__(256) parquet_levels_kernel(const __grid_consta
         __syncthreads();
         if (s_bad) break;
         const int n = s_n, e0 = s_emit, e1 = s_emit_end;
-        for (int k0 = e0; k0 < e1; k0 += 256) {
+        for (int k0 = e0; k0 < e1; k0 += kLevelThreads) {
             const int k = k0 + (int)threadIdx.x;
             ral_u32 X = 0;
             if (k < e1) {
@@ -906,13 +986,7 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const __grid_consta
     __shared__ ral_u32 s_base[256];
     __shared__ ral_u32 s_wsum[8];
     const int item = P.item_lo + (int)blockIdx.x;
-    int a = P.page_lo, b = P.page_hi - 1;  // the last page whose first item is at or before this one
-    while (a < b) {
-        const int m = (a + b + 1) >> 1;
-        if (P.pages[m].item0 <= item) a = m;
-        else b = m - 1;
-    }
-    const ParquetPage pg = P.pages[a];
+    const ParquetPage pg = P.pages[ral_pq_page_of(P, item)];
     const ParquetColumnOut col = P.out[pg.column];
     const int w = col.width;
     const int rel0 = (item - pg.item0) * kParquetItemRows;
@@ -924,65 +998,23 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const __grid_consta
         // a dictionary-encoded required page: row r's entry is idx[idx0 + r] (checked in range)
         const uint8_t* const dict = (const uint8_t*)pg.dict;
         const uint32_t* const ix = P.idx + pg.idx0;
-        for (int r = rel0 + (int)threadIdx.x; r < rel1; r += 256) {
-            const uint32_t k = ix[r];  // in range unless the page was malformed (then reported)
-            unsigned long long x = 0;
-            if (k < (uint32_t)pg.dict_count) x = ral_pq_value(dict, k, w);
-            ral_pq_store(col.data, pg.row_start + r, w, x);
+        // four rows at a time: their index loads, then their entries' loads, are in flight together
+        for (int r0 = rel0 + (int)threadIdx.x; r0 < rel1; r0 += 1024) {
+            uint32_t k[4];
+            unsigned long long x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) k[u] = r0 + 256 * u < rel1 ? ix[r0 + 256 * u] : 0xffffffffu;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)  // in range unless the page was malformed (then reported)
+                x[u] = k[u] < (uint32_t)pg.dict_count ? ral_pq_value(dict, k[u], w) : 0ull;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (r0 + 256 * u < rel1) ral_pq_store(col.data, pg.row_start + r0 + 256 * u, w, x[u]);
         }
         return;
     }
     if (!pg.optional) {
-        // Every row has its value (the page's length is checked on the host).  The lanes of a
-        // warp take consecutive rows: each loads the aligned word where its value starts and
-        // takes the next word from the lane after it (the last lane of the run loads it), so a
-        // warp reads one contiguous aligned span whatever the values' alignment.
-        const uintptr_t va = (uintptr_t)vals;
-        if (w == 8) {
-            // 16-byte words: lane l takes rows 2m, 2m + 1 (m = the warp's pair + l), bytes
-            // [s + 16m, s + 16m + 16) past the aligned base: word m and, when s > 0, word m + 1
-            // from the next lane (the last lane of the run loads it, when its values reach it)
-            const int s16 = (int)(va & 15);
-            const int k = s16 >> 2, f = (s16 & 3) * 8;
-            const uint4* q = reinterpret_cast<const uint4*>(va - s16);
-            unsigned long long* out = reinterpret_cast<unsigned long long*>(col.data) + pg.row_start;
-#pragma unroll 2
-            for (int m0 = (rel0 >> 1) + 32 * warp; 2 * m0 < rel1; m0 += 256) {
-                const int m = m0 + lane;
-                const int r = 2 * m;
-                const bool in = r < rel1;
-                const uint4 a = in ? q[m] : make_uint4(0u, 0u, 0u, 0u);
-                uint4 b;
-                b.x = __shfl_down_sync(0xffffffffu, a.x, 1);
-                b.y = __shfl_down_sync(0xffffffffu, a.y, 1);
-                b.z = __shfl_down_sync(0xffffffffu, a.z, 1);
-                b.w = __shfl_down_sync(0xffffffffu, a.w, 1);
-                const bool two = r + 1 < rel1;
-                if (in && (lane == 31 || r + 2 >= rel1) && s16 + (two ? 16 : 8) > 16) b = q[m + 1];
-                ral_u32 o0, o1, o2, o3;
-                switch (k) {  // uniform over the page
-                case 0: o0 = a.x; o1 = a.y; o2 = a.z; o3 = a.w; if (f) { o0 = __funnelshift_r(a.x, a.y, f); o1 = __funnelshift_r(a.y, a.z, f); o2 = __funnelshift_r(a.z, a.w, f); o3 = __funnelshift_r(a.w, b.x, f); } break;
-                case 1: o0 = __funnelshift_r(a.y, a.z, f); o1 = __funnelshift_r(a.z, a.w, f); o2 = __funnelshift_r(a.w, b.x, f); o3 = __funnelshift_r(b.x, b.y, f); break;
-                case 2: o0 = __funnelshift_r(a.z, a.w, f); o1 = __funnelshift_r(a.w, b.x, f); o2 = __funnelshift_r(b.x, b.y, f); o3 = __funnelshift_r(b.y, b.z, f); break;
-                default: o0 = __funnelshift_r(a.w, b.x, f); o1 = __funnelshift_r(b.x, b.y, f); o2 = __funnelshift_r(b.y, b.z, f); o3 = __funnelshift_r(b.z, b.w, f); break;
-                }
-                if (in) out[r] = (unsigned long long)o1 << 32 | o0;
-                if (two) out[r + 1] = (unsigned long long)o3 << 32 | o2;
-            }
-        } else {
-            const int sh = (int)(va & 3) * 8;
-            const ral_u32* q = reinterpret_cast<const ral_u32*>(va - (va & 3));
-            ral_u32* out = reinterpret_cast<ral_u32*>(col.data) + pg.row_start;
-#pragma unroll 4
-            for (int r0 = rel0 + 32 * warp; r0 < rel1; r0 += 256) {
-                const int r = r0 + lane;
-                const bool in = r < rel1;
-                const ral_u32 lo = in ? q[r] : 0u;
-                ral_u32 nx = __shfl_down_sync(0xffffffffu, lo, 1);
-                if (sh && in && (lane == 31 || r + 1 >= rel1)) nx = q[r + 1];
-                if (in) out[r] = sh ? (lo >> sh) | (nx << (32 - sh)) : lo;
-            }
-        }
+        if (!P.plain_done) ral_pq_plain_rows(pg, col, rel0, rel1, threadIdx.x);
         return;
     }
     // PLAIN values, or a dictionary's entries through the present rows' indices
@@ -1018,21 +1050,31 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const __grid_consta
     s_base[threadIdx.x] = before + incl - c;
     __syncthreads();
     const int64_t base = (int64_t)P.item_base[item];
-    // each warp takes one word (32 rows) per step
-    for (int t = warp; t * 32 < rel1 - rel0; t += 8) {
-        const int r = rel0 + 32 * t + lane;
-        if (r >= rel1) break;
-        const ral_u32 Xw = s_word[t];
-        unsigned long long x = 0;
-        if ((Xw >> lane) & 1u) {
-            const int64_t vi = base + s_base[t] + __popc(Xw & ((1u << lane) - 1u));
-            if (pg.dict_count > 0) {
-                const uint32_t k = ix[vi];
-                if (k < (uint32_t)pg.dict_count) x = ral_pq_value(dict, k, w);
-            }
-            else if (vi < nvals) x = ral_pq_value(vals, vi, w);
+    // each warp takes four words (of 32 rows) per step, their loads in flight together
+    for (int t0 = warp; t0 * 32 < rel1 - rel0; t0 += 32) {
+        int64_t vi[4];  // the row's value, or -1
+        unsigned long long x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int t = t0 + 8 * u, r = rel0 + 32 * t + lane;
+            const ral_u32 Xw = r < rel1 ? s_word[t] : 0u;
+            vi[u] = (Xw >> lane) & 1u ? base + s_base[t] + __popc(Xw & ((1u << lane) - 1u)) : -1;
         }
-        ral_pq_store(col.data, pg.row_start + r, w, x);
+        if (pg.dict_count > 0) {
+            uint32_t k[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) k[u] = vi[u] >= 0 ? ix[vi[u]] : 0xffffffffu;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = k[u] < (uint32_t)pg.dict_count ? ral_pq_value(dict, k[u], w) : 0ull;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = vi[u] >= 0 && vi[u] < nvals ? ral_pq_value(vals, vi[u], w) : 0ull;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int r = rel0 + 32 * (t0 + 8 * u) + lane;
+            if (r < rel1) ral_pq_store(col.data, pg.row_start + r, w, x[u]);
+        }
     }
 }
 
@@ -1450,7 +1492,8 @@ cudaError_t launch_prepare_jobs(const PrepareJob* jobs, int32_t n_jobs, cudaStre
 
 cudaError_t launch_parquet_levels(const ParquetDecodeParams& p, cudaStream_t st) {
     if (p.page_hi <= p.page_lo) return cudaSuccess;
-    parquet_levels_kernel<<<p.page_hi - p.page_lo, 256, 0, st>>>(p);
+    const int items = p.item_hi - p.item_lo, per = kLevelThreads / 256;
+    parquet_levels_kernel<<<p.page_hi - p.page_lo + (items + per - 1) / per, kLevelThreads, 0, st>>>(p);
     note_launch();
     return cudaGetLastError();
 }

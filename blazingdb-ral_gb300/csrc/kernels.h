@@ -120,6 +120,7 @@ struct ParquetDecodeParams {
     uint32_t* idx;               // dictionary indices of the present rows of dictionary-encoded pages
     int32_t page_lo, page_hi;    // the pages of this launch
     int32_t item_lo, item_hi;    // their items
+    int32_t plain_done;          // the levels kernel's launch has written the required PLAIN pages' values
 };
 // One Snappy-compressed page body (a Parquet page of a SNAPPY column chunk): `prefix` raw bytes
 // (a v2 page's levels, stored uncompressed before the values) are copied from src - prefix, then
@@ -169,7 +170,8 @@ cudaError_t launch_copy_headers(const HeaderJob* jobs, int32_t n, unsigned long 
 // first 4 bytes of their decompressed data, and their values' offset after it.
 cudaError_t launch_parquet_level_lengths(const ParquetDecodeParams& p, cudaStream_t st);
 // Optional pages of [page_lo, page_hi): validity bits from the definition levels, each item's
-// first value index in item_base, the present rows in status[1 + column].
+// first value index in item_base, the present rows in status[1 + column].  Also the values of the
+// required PLAIN pages among them.
 cudaError_t launch_parquet_levels(const ParquetDecodeParams& p, cudaStream_t st);
 // Dictionary-encoded pages of [page_lo, page_hi): the index of every present row (RLE / bit-packed
 // hybrid of the page's bit width) into idx, checked against the dictionary's size.  After

@@ -508,6 +508,7 @@ int parquet_scan_filter(const uint8_t* file, int64_t n, const int32_t* projectio
             dict |= pages[k].dict_count > 0;
             lens |= pages[k].levels < 0;
         }
+        dp.plain_done = opt ? 1 : 0;
         if (lens && check_cuda(launch_parquet_level_lengths(dp, st), "Parquet level lengths")) return kCudaError;
         if (opt && check_cuda(launch_parquet_levels(dp, st), "Parquet definition levels")) return kCudaError;
         if (dict && check_cuda(launch_parquet_dict_indices(dp, st), "Parquet dictionary indices")) return kCudaError;
