@@ -517,10 +517,17 @@ int enqueue_prepared(const PreparedFilter& pf, gdf_column* const* frame, gdf_col
         __atomic_store_n(&area->hmap[0], 0ull, __ATOMIC_RELEASE);  // no earlier call's tag can match
     } else {
         if (grid_call) grid_call->used = false;
-        cudaMemsetAsync(scratch, 0, (size_t)prepared_scratch_words(pf, n) * 8, st);
         // output masks are assembled with OR at the edges of each warp's range: start from zero
-        for (int q = 0; q < NO; q++)
-            if (spec.outputs[q].has_valid) cudaMemsetAsync(outs[q]->valid, 0, (size_t)((n + obase + 31) / 32) * 4, st);
+        ZeroList zero{};
+        zero.add(scratch, 2 * prepared_scratch_words(pf, n));
+        for (int q = 0; q < NO; q++) {
+            if (zero.n == kMaxZeroList) {
+                if (int e = check_cuda(launch_zero_list(zero, st), "filter scratch")) return e;
+                zero.n = 0;
+            }
+            if (spec.outputs[q].has_valid) zero.add(outs[q]->valid, (n + obase + 31) / 32);
+        }
+        if (int e = check_cuda(launch_zero_list(zero, st), "filter scratch")) return e;
     }
 
     std::vector<uint64_t> slots(L.total, 0);

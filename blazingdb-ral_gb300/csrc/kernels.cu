@@ -1483,6 +1483,24 @@ cudaError_t launch_copy_headers(const HeaderJob* jobs, int32_t n, unsigned long 
     return cudaGetLastError();
 }
 
+// In place of a memset per scratch area and output mask before a filter or a text scan, some 2 us each, one
+// after the other (9M rows of six columns with nulls, half of them kept: 183 -> 161 us; the masks of a 20M-line text scan 799 -> 786 us).
+__global__ void __launch_bounds__(256) zero_list_kernel(const __grid_constant__ ZeroList list) {
+    ral_fill(CopyJob{nullptr, (uint8_t*)list.p[blockIdx.y], 4 * list.words[blockIdx.y]}, 0u,
+             (int64_t)blockIdx.x * 256 + threadIdx.x, (int64_t)gridDim.x * 256);
+}
+
+cudaError_t launch_zero_list(const ZeroList& list, cudaStream_t st) {
+    if (list.n <= 0) return cudaSuccess;
+    int64_t most = 0;
+    for (int k = 0; k < list.n; k++) most = std::max(most, list.words[k]);
+    // 4 of the 16-byte words a thread, up to the device's threads for all ranges together
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((most + 4095) / 4096, (152 * 8 + list.n - 1) / list.n));
+    zero_list_kernel<<<dim3((unsigned)blocks, (unsigned)list.n), 256, 0, st>>>(list);
+    note_launch();
+    return cudaGetLastError();
+}
+
 cudaError_t launch_prepare_jobs(const PrepareJob* jobs, int32_t n_jobs, cudaStream_t st) {
     if (n_jobs <= 0) return cudaSuccess;
     prepare_jobs_kernel<<<n_jobs, 256, 0, st>>>(jobs);

@@ -158,6 +158,19 @@ struct CopyList {
     int32_t n;
 };
 cudaError_t launch_copy_list(const CopyList& list, cudaStream_t st);
+// Zeroes up to kMaxZeroList ranges of device memory (4-byte aligned, whole 4-byte words) in one launch.
+constexpr int kMaxZeroList = 72;
+struct ZeroList {
+    void* p[kMaxZeroList];
+    int64_t words[kMaxZeroList];  // of 4 bytes
+    int32_t n;
+    void add(void* at, int64_t w) {
+        if (w <= 0) return;
+        p[n] = at;
+        words[n++] = w;
+    }
+};
+cudaError_t launch_zero_list(const ZeroList& list, cudaStream_t st);
 // words[k] (at most 67) 8-byte words from src[k], device memory, to dst + 67 k, page-locked host memory: the
 // finished requests' headers of a served wave, one launch in place of a copy each.
 struct HeaderJob {

@@ -295,8 +295,8 @@ int64_t range_bytes(int64_t n, int64_t cap) {
 // Synchronous on st.
 int scan_piece(const PreparedScan& ps, const char* data, int64_t n, char delim, char term, int64_t from,
                int32_t skip_rows, gdf_column* const* outs, int NP, int64_t row0, int64_t cap, cudaStream_t st,
-               int64_t& kept, std::vector<int64_t>& valid) {
-    if (n <= from) return kSuccess;
+               int64_t& kept, std::vector<int64_t>& valid, ZeroList zero = {}) {
+    if (n <= from) return check_cuda(launch_zero_list(zero, st), "text scan masks");
     const ParamLayout& L = ps.gk.layout;
     const int64_t head = (int64_t)((uintptr_t)data & 15);
     const int64_t rb = range_bytes(n - from, cap);
@@ -308,7 +308,8 @@ int scan_piece(const PreparedScan& ps, const char* data, int64_t n, char delim, 
     StreamBuffer scratch(st), list(st);
     if (int e = scratch.alloc((size_t)(header + ranges) * 8)) return e;
     if (int e = list.alloc((size_t)listed * 8)) return e;
-    cudaMemsetAsync(scratch.p, 0, (size_t)(header + ranges) * 8, st);
+    zero.add(scratch.p, 2 * (header + ranges));
+    if (int e = check_cuda(launch_zero_list(zero, st), "text scan scratch")) return e;
     if (skip_rows > 0)
         if (int e = skip_lines(data + from, n - from, term, skip_rows, (unsigned long long*)scratch.p + header - 1, st))
             return e;
@@ -394,11 +395,11 @@ int text_scan_filter(const char* data, int64_t n, char delim, char term, int32_t
     const int NP = n_proj;
     cudaStream_t st = cudaStreamPerThread;
     keep_pool_memory();
-    for (int q = 0; q < NP; q++)
-        if (cap > 0) cudaMemsetAsync(outs[q]->valid, 0, (size_t)((cap + 31) / 32) * 4, st);
+    ZeroList zero{};
+    for (int q = 0; q < NP; q++) zero.add(outs[q]->valid, (cap + 31) / 32);
     int64_t kept = 0;
     std::vector<int64_t> valid(NP, 0);
-    if (int e = scan_piece(*ps, data, n, delim, term, 0, skip_rows, outs, NP, 0, cap, st, kept, valid)) return e;
+    if (int e = scan_piece(*ps, data, n, delim, term, 0, skip_rows, outs, NP, 0, cap, st, kept, valid, zero)) return e;
     set_outputs(outs, NP, kept, valid, n_out);
     return kSuccess;
 }
