@@ -78,15 +78,11 @@ RAL_FI float ral_d2f(double d) { return __double2float_rn(d); }
 #ifndef RAL_SOFT_TRIG
 #define RAL_SOFT_TRIG 1
 #endif
-// Item functions call these (they are the dispatch kernel's; bits as below and above)
+// Item functions call the dispatch kernel's ral_shared_* (declared before this prelude; the same bits)
 #if defined(RAL_SHARED_OPS)
-extern "C" __device__ double ral_shared_ddiv(double a, double b);
-extern "C" __device__ ral_i64 ral_shared_divi(ral_i64 a, ral_i64 b);
-extern "C" __device__ ral_i64 ral_shared_modi(ral_i64 a, ral_i64 b);
 RAL_FI double ral_ddiv(double a, double b) { return ral_shared_ddiv(a, b); }
 #endif
 #if RAL_SOFT_TRIG && defined(RAL_SHARED_OPS)
-extern "C" __device__ double ral_shared_trig(double x, int want_cos);
 RAL_FI double ral_dsin(double x) { return ral_shared_trig(x, 0); }
 RAL_FI double ral_dcos(double x) { return ral_shared_trig(x, 1); }
 #elif RAL_SOFT_TRIG

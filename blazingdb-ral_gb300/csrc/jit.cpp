@@ -72,7 +72,12 @@ const std::string& soft_fp_define(bool soft) {
 }
 
 std::string full_source(const GeneratedKernel& gk) {
-    return std::string(gk.shared_ops ? "#define RAL_SHARED_OPS\n" : "") + trig_define() + soft_fp_define(gk.soft_fp) +
+    static const std::string shared =
+        "#define RAL_SHARED_OPS\nextern \"C\" __device__ double ral_shared_trig(double x, int want_cos);\n"
+        "extern \"C\" __device__ double ral_shared_ddiv(double a, double b);\n"
+        "extern \"C\" __device__ long long ral_shared_divi(long long a, long long b);\n"
+        "extern \"C\" __device__ long long ral_shared_modi(long long a, long long b);\n";
+    return (gk.shared_ops ? shared : std::string()) + trig_define() + soft_fp_define(gk.soft_fp) +
            std::string(ral_prelude_source) + "\n" + gk.source;
 }
 
