@@ -747,6 +747,17 @@ __device__ __forceinline__ int ral_pq_page_of(const ParquetDecodeParams& P, int 
     return a;
 }
 
+// A block beyond the pages' own of a 1024-thread kernel: the items 4 k .. 4 k + 3 of every plain_every-th one,
+// of which it writes those of required PLAIN pages.
+__device__ __forceinline__ void ral_pq_plain_block(const ParquetDecodeParams& P, int k) {
+    const int item = P.item_lo + (4 * k + (int)(threadIdx.x >> 8)) * P.plain_every;
+    if (item >= P.item_hi) return;
+    const ParquetPage pg = P.pages[ral_pq_page_of(P, item)];
+    if (pg.optional || pg.dict_count > 0) return;
+    const int rel0 = (item - pg.item0) * kParquetItemRows;
+    ral_pq_plain_rows(pg, P.out[pg.column], rel0, min(rel0 + kParquetItemRows, pg.rows), threadIdx.x & 255);
+}
+
 // One block per optional page.  The run headers form a chain of which only the start is known.  Every
 // byte of a 12 KiB window of the stream is read as if a header started there, by all threads, which
 // leaves the bytes to the next one; thread 0 then only adds hops (some 45 cycles a run), and the runs it
@@ -766,12 +777,7 @@ __global__ void __launch_bounds__(kLevelThreads) parquet_levels_kernel(const __g
     __shared__ int s_n, s_new, s_bad, s_emit, s_emit_end, s_done;
     __shared__ long long s_pos, s_w[kLevelThreads / 32];
     if ((int)blockIdx.x >= P.page_hi - P.page_lo) {
-        const int item = P.item_lo + ((int)blockIdx.x - (P.page_hi - P.page_lo)) * (kLevelThreads / 256) + (int)(threadIdx.x >> 8);
-        if (item >= P.item_hi) return;
-        const ParquetPage pg = P.pages[ral_pq_page_of(P, item)];
-        if (pg.optional || pg.dict_count > 0) return;
-        const int rel0 = (item - pg.item0) * kParquetItemRows;
-        ral_pq_plain_rows(pg, P.out[pg.column], rel0, min(rel0 + kParquetItemRows, pg.rows), threadIdx.x & 255);
+        ral_pq_plain_block(P, (int)blockIdx.x - (P.page_hi - P.page_lo));
         return;
     }
     const ParquetPage pg = P.pages[P.page_lo + blockIdx.x];
@@ -1014,7 +1020,7 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const __grid_consta
         return;
     }
     if (!pg.optional) {
-        if (!P.plain_done) ral_pq_plain_rows(pg, col, rel0, rel1, threadIdx.x);
+        if (P.plain_every == 0 || (item - P.item_lo) % P.plain_every) ral_pq_plain_rows(pg, col, rel0, rel1, threadIdx.x);
         return;
     }
     // PLAIN values, or a dictionary's entries through the present rows' indices
@@ -1103,6 +1109,10 @@ __global__ void __launch_bounds__(kDictThreads) parquet_dict_index_kernel(const 
     __shared__ unsigned char s_kind[kPqRuns];
     __shared__ int s_n, s_bad, s_done;
     __shared__ long long s_pos, s_rem;  // the stream offset reached, and the groups left of the run it is in
+    if ((int)blockIdx.x >= P.page_hi - P.page_lo) {
+        ral_pq_plain_block(P, ((int)blockIdx.x - (P.page_hi - P.page_lo)) * kDictSlices + (int)blockIdx.y);
+        return;
+    }
     const int p = P.page_lo + (int)blockIdx.x;
     const ParquetPage pg = P.pages[p];
     if (pg.dict_count <= 0 || pg.rows <= 0) return;
@@ -1259,7 +1269,9 @@ __global__ void __launch_bounds__(kDictThreads) parquet_dict_index_kernel(const 
 
 cudaError_t launch_parquet_dict_indices(const ParquetDecodeParams& p, cudaStream_t st) {
     if (p.page_hi <= p.page_lo) return cudaSuccess;
-    parquet_dict_index_kernel<<<dim3(p.page_hi - p.page_lo, kDictSlices), kDictThreads, 0, st>>>(p);
+    const int items = p.plain_every > 1 ? (p.item_hi - p.item_lo + p.plain_every - 1) / p.plain_every : 0;
+    parquet_dict_index_kernel<<<dim3(p.page_hi - p.page_lo + (items + 4 * kDictSlices - 1) / (4 * kDictSlices), kDictSlices),
+                                kDictThreads, 0, st>>>(p);
     note_launch();
     return cudaGetLastError();
 }
@@ -1510,8 +1522,7 @@ cudaError_t launch_prepare_jobs(const PrepareJob* jobs, int32_t n_jobs, cudaStre
 
 cudaError_t launch_parquet_levels(const ParquetDecodeParams& p, cudaStream_t st) {
     if (p.page_hi <= p.page_lo) return cudaSuccess;
-    const int items = p.item_hi - p.item_lo, per = kLevelThreads / 256;
-    parquet_levels_kernel<<<p.page_hi - p.page_lo + (items + per - 1) / per, kLevelThreads, 0, st>>>(p);
+    parquet_levels_kernel<<<p.page_hi - p.page_lo + (p.item_hi - p.item_lo + 3) / 4, kLevelThreads, 0, st>>>(p);
     note_launch();
     return cudaGetLastError();
 }

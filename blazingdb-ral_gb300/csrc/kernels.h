@@ -120,7 +120,9 @@ struct ParquetDecodeParams {
     uint32_t* idx;               // dictionary indices of the present rows of dictionary-encoded pages
     int32_t page_lo, page_hi;    // the pages of this launch
     int32_t item_lo, item_hi;    // their items
-    int32_t plain_done;          // the levels kernel's launch has written the required PLAIN pages' values
+    // The required PLAIN pages' values wait for nothing: all of them (1) are written beside the levels kernel, or
+    // every plain_every-th item's beside the dictionary indices' kernel; 0: all by the values kernel.
+    int32_t plain_every;
 };
 // One Snappy-compressed page body (a Parquet page of a SNAPPY column chunk): `prefix` raw bytes
 // (a v2 page's levels, stored uncompressed before the values) are copied from src - prefix, then

@@ -48,6 +48,12 @@ struct DevBuf {
     int alloc(size_t bytes) { return check_cuda(cudaMallocAsync(&p, std::max<size_t>(bytes, 16), st), "cudaMallocAsync"); }
 };
 
+// Every how many of the required PLAIN items are written beside the dictionary indices' kernel, the others
+// beside the dictionary pages' values: both kernels work on device memory while the link brings PLAIN pages (6M
+// and 20M rows of required columns, three of four with dictionaries: 510 and 1464 us; every 2nd 510 and
+// 1460, every 8th 532 and 1537, all 545 and 1581, none 541 and 1591).
+constexpr int kPlainEvery = 4;
+
 // Pages go to the device in batches of about this many bytes (RAL_PARQUET_BATCH_BYTES overrides),
 // each copied while the one before it is decoded.
 int64_t batch_bytes() {
@@ -508,7 +514,7 @@ int parquet_scan_filter(const uint8_t* file, int64_t n, const int32_t* projectio
             dict |= pages[k].dict_count > 0;
             lens |= pages[k].levels < 0;
         }
-        dp.plain_done = opt ? 1 : 0;
+        dp.plain_every = opt ? 1 : dict ? kPlainEvery : 0;
         if (lens && check_cuda(launch_parquet_level_lengths(dp, st), "Parquet level lengths")) return kCudaError;
         if (opt && check_cuda(launch_parquet_levels(dp, st), "Parquet definition levels")) return kCudaError;
         if (dict && check_cuda(launch_parquet_dict_indices(dp, st), "Parquet dictionary indices")) return kCudaError;
