@@ -85,7 +85,7 @@ def batch_mix_meta(n_programs, seed):
 
 
 def floor_table_from_ncu(csv_path, n_programs, seed, cap):
-    """profiles/batch_mix_fp64.json from an ncu CSV of the mix's plain calls over tables capped at
+    """profiles/batch_mix_counters.json from an ncu CSV of the mix's plain calls over tables capped at
     `cap` rows (one ral_eval launch per program, in program order): FP64 and all thread
     instructions per row of every program."""
     import csv
@@ -122,7 +122,7 @@ def batch_floor(table, sm_mhz, peak_gbs):
             "floor_ms": max(sum(fp), sum(hb)) * 1e3,
             "per_program_floor_ms": sum(max(a, b) for a, b in zip(fp, hb)) * 1e3,
             "fp64_rate": f"{FP64_PER_CLOCK_PER_SM} per clock per SM x {SMS} SMs x {sm_mhz:.0f} MHz",
-            "source": "profiles/batch_mix_fp64.json"}
+            "source": "profiles/batch_mix_counters.json"}
 
 
 class ClockSampler:
@@ -456,7 +456,7 @@ def workload_config(workload, n, selectivity, world=1):
                         + ", 1Mi-row row groups, in page-locked host memory",
                "scan": f"BindableTableScan projects={W.TEXT_PROJECTIONS}", "filter": "TPC-H Q6's conditions",
                "fused": "the projected pages read in place from page-locked host memory"
-                        + (", dictionary indices decoded by one block per page" if dictionary else "")
+                        + (", dictionary indices decoded by eight blocks per page" if dictionary else "")
                         + ", the page-value kernel (a block per 8192-row item of a page), then the fused filter kernel",
                "l2": "decoded columns (560 MB at 20M rows) exceed L2; no flush"}
     elif workload == "scan_filter":
@@ -465,7 +465,7 @@ def workload_config(workload, n, selectivity, world=1):
                "table": "lineitem-like '|'-delimited text: orderkey int64, partkey int32, quantity int32, "
                         "extendedprice float64, discount float64, tax float32, shipdate date64, commitdate date32",
                "scan": f"BindableTableScan projects={W.TEXT_PROJECTIONS}", "filter": "TPC-H Q6's conditions",
-               "fused": "parse + filter + compaction in one kernel (after a line index)",
+               "fused": "one kernel finds the lines, evaluates the condition and lists the kept ones, one parses their projected fields",
                "l2": "text (1.3 GB at 20M rows) exceeds L2; no flush"}
     elif workload == "plain_vm":
         cfg = {"workload": "plain_vm", "rows": n, "filter": "((c2>=24 AND c1<0.05) OR c0%7=3) AND c3<1200",
@@ -1403,7 +1403,7 @@ def batched_capped(R, progs, cap, stream, plain_steps):
 def batched_floor_block(args, clocks, ms_per_step, plain):
     """The floor of the default mix from the committed per-program counters, at the clock measured
     during the timed region; None for another mix."""
-    p = os.path.join(ROOT, "profiles", "batch_mix_fp64.json")
+    p = os.path.join(ROOT, "profiles", "batch_mix_counters.json")
     if not os.path.exists(p) or args.max_rows or args.programs != 256 or args.seed != 20261203:
         return None
     table = json.load(open(p))
@@ -1770,7 +1770,7 @@ def main():
         args.warmup = 3
     if args.floor_from_ncu:
         table = floor_table_from_ncu(args.floor_from_ncu, args.programs, args.seed, args.max_rows or 200_000)
-        with open(os.path.join(ROOT, "profiles", "batch_mix_fp64.json"), "w") as f:
+        with open(os.path.join(ROOT, "profiles", "batch_mix_counters.json"), "w") as f:
             json.dump(table, f, indent=0)
         print(json.dumps(batch_floor(table, 2070.0, load_peaks()[0])))
         return
