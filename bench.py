@@ -1752,7 +1752,7 @@ def main():
     ap.add_argument("--no-autotune", action="store_true")
     ap.add_argument("--max-rows", type=int, default=0, help="batched: cap every table (profiling captures)")
     ap.add_argument("--floor-from-ncu", default=None,
-                    help="batched: write profiles/batch_mix_fp64.json from an ncu CSV of the capped plain calls "
+                    help="batched: write profiles/batch_mix_counters.json from an ncu CSV of the capped plain calls "
                          "(no GPU needed) and exit")
     ap.add_argument("--capped-rows", type=int, default=1_000_000,
                     help="batched: also compare batch and plain calls over the first N rows of every table")
