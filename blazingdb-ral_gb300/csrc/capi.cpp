@@ -909,33 +909,51 @@ int ral_server_copy_result(ral_server* server, int64_t request_id, gdf_column* c
         if (!server || !out_columns || num_outputs <= 0) return set_error(kInvalidArgument, "bad argument");
         std::vector<gdf_column> src(num_outputs);
         if (int e = server->s.result(request_id, src.data(), num_outputs)) return e;
+        for (int o = 0; o < num_outputs; o++) {
+            const gdf_column* d = out_columns[o];
+            if (!d) return set_error(kInvalidArgument, "null out column");
+            if (d->dtype != src[o].dtype) return set_error(kInvalidArgument, "out column has the wrong dtype");
+            if ((d->valid != nullptr) != (src[o].valid != nullptr))
+                return set_error(kInvalidArgument, "out column mask presence differs from the query's");
+            if (src[o].size > 0 && !d->data) return set_error(kInvalidArgument, "out column without data");
+        }
         cudaStream_t st = cudaStreamPerThread;
+        int dev = 0;
+        if (int e = check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return e;
+        // One kernel copies what lies on the server's device, where that is the current one; other buffers
+        // (another device's, host memory) are the copy engine's, which reaches them all and refuses the rest.
+        const bool here = dev == server->s.device();
         CopyList list;
         list.n = 0;
         auto add = [&](const void* s, void* d, size_t bytes) -> int {
             if (!bytes) return kSuccess;
+            cudaPointerAttributes at{};
+            if (here && cudaPointerGetAttributes(&at, d) != cudaSuccess) cudaGetLastError();
+            if (at.type != cudaMemoryTypeDevice || at.device != dev)
+                return check_cuda(cudaMemcpyAsync(d, s, bytes, cudaMemcpyDeviceToDevice, st), "copy of a served result");
             list.job[list.n++] = CopyJob{(const uint8_t*)s, (uint8_t*)d, (int64_t)bytes};
             if (list.n < kMaxCopyList) return kSuccess;
             const cudaError_t e = launch_copy_list(list, st);
             list.n = 0;
             return check_cuda(e, "copy of a served result");
         };
-        for (int o = 0; o < num_outputs; o++) {
+        int rc = kSuccess;
+        for (int o = 0; o < num_outputs && !rc; o++) {
             gdf_column* d = out_columns[o];
-            if (!d) return set_error(kInvalidArgument, "null out column");
-            if (d->dtype != src[o].dtype) return set_error(kInvalidArgument, "out column has the wrong dtype");
-            if ((d->valid != nullptr) != (src[o].valid != nullptr))
-                return set_error(kInvalidArgument, "out column mask presence differs from the query's");
-            const size_t nb = (size_t)src[o].size * gdf_dtype_size(src[o].dtype);
-            if (int e = add(src[o].data, d->data, nb)) return e;
-            if (src[o].valid)
-                if (int e = add(src[o].valid, d->valid, ((size_t)src[o].size + 7) / 8)) return e;
-            d->size = src[o].size;
-            d->null_count = src[o].null_count;
+            rc = add(src[o].data, d->data, (size_t)src[o].size * gdf_dtype_size(src[o].dtype));
+            if (!rc && src[o].valid) rc = add(src[o].valid, d->valid, ((size_t)src[o].size + 7) / 8);
         }
-        if (list.n)
-            if (int e = check_cuda(launch_copy_list(list, st), "copy of a served result")) return e;
-        return check_cuda(cudaStreamSynchronize(st), "copy of a served result");
+        if (!rc && list.n) rc = check_cuda(launch_copy_list(list, st), "copy of a served result");
+        if (rc) {
+            cudaStreamSynchronize(st);  // nothing is written after the call
+            return rc;
+        }
+        if (int e = check_cuda(cudaStreamSynchronize(st), "copy of a served result")) return e;
+        for (int o = 0; o < num_outputs; o++) {
+            out_columns[o]->size = src[o].size;
+            out_columns[o]->null_count = src[o].null_count;
+        }
+        return (int)kSuccess;
     });
 }
 

@@ -107,6 +107,7 @@ public:
                   double* makespan_s);
     int stop();
     ServerStats stats() const;
+    int device() const { return device_; }
     double now() const;
 
 private:
