@@ -42,7 +42,8 @@ std::string tune_path() {
     return dir + "/autotune.json";
 }
 
-// The table is a flat JSON object {"key": [J, U, ms, S], ...}; keys contain no quotes.
+// The table is a flat JSON object {"key@version": [J, U, ms, S], ...}; keys contain no quotes.  Entries of
+// other versions are carried along for the builds that wrote them.
 void load_tune_locked() {
     if (g_tune_loaded) return;
     g_tune_loaded = true;
@@ -152,6 +153,24 @@ std::string tune_key(const Program& p, int G) {
            std::to_string(bucket(std::max(1, nin)));
 }
 
+// A program's entry in the table.  Which shape wins depends on the code of the items: when their divisions and
+// sin / cos moved to shared functions, entries that had chosen the integer-pipe forms (29 of 34 keys of
+// the 256-program mix) became the slower choice (9.8 ms against 6.4 with tables of up to 1M rows).  So an
+// entry counts only for the code it was timed with: the device prelude, the dispatcher with the shared
+// functions, and the item generator's version (raised when generate_batch_item's code changes).
+std::string table_key(const Program& p, int G) {
+    static const std::string version = [] {
+        constexpr int kItemCode = 1;
+        const std::string code = std::string(jit_prelude()) + generate_batch_dispatch({}, 0, 1).source + std::to_string(kItemCode);
+        uint64_t h = 1469598103934665603ull;
+        for (const char c : code) h = (h ^ (unsigned char)c) * 1099511628211ull;
+        char hex[24];
+        snprintf(hex, sizeof hex, "@%016llx", (unsigned long long)h);
+        return std::string(hex);
+    }();
+    return tune_key(p, G) + version;
+}
+
 Shape tuned_shape(const Program& p, int G) {
     Shape s;
     s.G = G;
@@ -160,7 +179,7 @@ Shape tuned_shape(const Program& p, int G) {
     s.threads = 256;
     std::lock_guard<std::mutex> lock(g_tune_mu);
     load_tune_locked();
-    auto it = g_tune.find(tune_key(p, G));
+    auto it = g_tune.find(table_key(p, G));
     if (it != g_tune.end()) {
         s.J = it->second.J;
         s.unroll = it->second.U;
@@ -177,7 +196,7 @@ void record_tuned_shape(const Program& p, int G, int J, int U, bool soft, double
     te.U = U;
     te.S = soft ? 1 : 0;
     te.ms = ms;
-    g_tune[tune_key(p, G)] = te;
+    g_tune[table_key(p, G)] = te;
     save_tune_locked();
 }
 
