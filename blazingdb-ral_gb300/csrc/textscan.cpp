@@ -121,11 +121,13 @@ std::mutex g_scan_mu;
 std::map<std::string, std::unique_ptr<PreparedScan>> g_scans;
 
 Shape text_scan_shape() {
-    // four warps a block, whose rings and bitmaps take 43 KB of shared memory: five blocks an SM
+    // four warps a block, whose rings and bitmaps take 39 KB of shared memory: five blocks an SM.  More warps
+    // would pass the 48 KB of a plain launch, so a larger T of RAL_SCAN_TUNE counts as 128.
     Shape s;
     s.threads = 128;
     s.min_blocks = 5;
     apply_shape_tune(s, std::getenv("RAL_SCAN_TUNE") ? std::getenv("RAL_SCAN_TUNE") : "");
+    s.threads = std::min(s.threads, 128);
     return s;
 }
 
