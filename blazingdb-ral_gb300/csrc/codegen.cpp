@@ -1974,12 +1974,15 @@ void emit_text_finders(std::ostream& os, const std::vector<int>& fields) {
         os << "    fe[" << at(f) << "] = d" << f << " < e ? d" << f << " : e;\n";
     }
     os << "}\n";
-    os << "RAL_FI void ral_fields_slow(const char* d, ral_i64 e, char delim, ral_i64* fs, ral_i64* fe) {\n";
+    // The line at d ends at its terminator or at e, less a '\r' before that; no byte after the last needed field
+    // is read (searched for its end first, by one warp and then by one lane, a line of 64 MB took 4.4 s; 0.26 ms).
+    os << "RAL_FI void ral_fields_slow(const char* d, ral_i64 e, char delim, char term, ral_i64* fs, ral_i64* fe) {\n";
     os << "#pragma unroll\n    for (int k = 0; k < " << fields.size() << "; ++k) { fs[k] = -1; fe[k] = -1; }\n";
     os << "    int f = 0;\n    ral_i64 p0 = 0;\n";
     os << "    for (ral_i64 p = 0;; ++p) {\n";
-    os << "        const bool end = p >= e;\n";
-    os << "        if (end || d[p] == delim) {\n";
+    os << "        const char c = p < e ? d[p] : term;\n";
+    os << "        const bool end = c == term || (c == '\\r' && (p + 1 >= e || d[p + 1] == term));\n";
+    os << "        if (end || c == delim) {\n";
     os << "            switch (f) {\n";
     for (size_t k = 0; k < fields.size(); k++)
         os << "            case " << fields[k] << ": fs[" << k << "] = p0; fe[" << k << "] = p; break;\n";
@@ -2026,6 +2029,10 @@ void emit_text_parse(std::ostream& os, const std::string& ind, gdf_dtype dt, con
     os << ind << "    " << v << " = ok ? " << val << " : " << (isf ? "0.0" : "0") << ";\n";
     os << ind << "}\n";
 }
+
+// A line's length in the kept-line list, where 65535 stands for a line past the ring, whose end is not
+// known: up to the text's end.
+std::string text_long_end() { return "    if (n == 65535) n = (const char*)P.s[1] + P.s[2] - ls;\n"; }
 
 // Column c's variables around a call of the out-of-line line parser: what it writes through references
 // are copies, so that the columns themselves stay in registers.
@@ -2104,12 +2111,12 @@ GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s)
                 os << "RAL_FI bool ral_keep(const RalParams& P, const ral_u32* tx, const ral_u32* db, ral_u32 s, ral_u32 e,\n"
                       "                     const char* ls, ral_u32& refused) {\n";
             else
-                os << "static __device__ __noinline__ ral_u32 ral_keep_long(const RalParams& P, const char* ls, ral_i64 n, char delim) {\n"
-                      "    ral_u32 refused = 0u;\n";
+                os << "static __device__ __noinline__ ral_u32 ral_keep_long(const RalParams& P, const char* ls, ral_i64 n) {\n"
+                      "    ral_u32 refused = 0u;\n" << text_long_end();
             const char* w = staged ? "ral_u32" : "ral_i64";
             if (!parts.f1.empty()) {
                 os << "    " << w << " fs[" << parts.f1.size() << "], fe[" << parts.f1.size() << "];\n";
-                os << (staged ? "    ral_fields(db, s, e, fs, fe);\n" : "    ral_fields_slow(ls, n, delim, fs, fe);\n");
+                os << (staged ? "    ral_fields(db, s, e, fs, fe);\n" : "    ral_fields_slow(ls, n, (char)(P.s[6] & 0xffu), (char)(P.s[6] >> 8), fs, fe);\n");
             }
             os << "    ral_u32 fv[" << std::max<size_t>(1, t.predicate_cols.size()) << "];\n";
             for (size_t c = 0; c < t.predicate_cols.size(); c++) {
@@ -2188,9 +2195,8 @@ GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s)
         for (int pass = 0;; ++pass) {
             ral_u32 total = 0;
             if (any_line) {
-                ral_i64 last_end = -1;  // where a line longer than the ring ends
                 // the queue: the position before the first line's start, then terminators; line j lies between
-                // entries j and j + 1 (16 bits: -1 wraps and comes back; 0xffff as an end is last_end)
+                // entries j and j + 1 (16 bits: -1 wraps and comes back; 0xffff as an end stands for one past the ring)
                 ral_u32 qh = 0, qt = 0;
                 __syncwarp();
                 if (base + first == start || R[(ral_i64)first - 1] == term) {
@@ -2229,19 +2235,7 @@ GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s)
                             } else if (off >= hi_r) {  // the text's last line has no terminator
                                 e = hi_r;
                             } else if (off >= RB + RAL_RING) {
-                                // longer than the ring: its end is searched, its bytes are read from global memory
-                                last_end = hi;
-                                for (ral_i64 p = base + off; p < hi; p += 512) {
-                                    const ral_i64 at = p + 16 * lane;
-                                    const ral_u32 n = at < hi ? (ral_u32)(hi - at < 16 ? hi - at : 16) : 0u;
-                                    const ral_u32 m = n ? ral_txv_eq16(ral_txv_load16(A + at, 0u, 0u, n), T4) & ((1u << n) - 1u) : 0u;
-                                    const ral_u32 b = __ballot_sync(0xffffffffu, m != 0u);
-                                    if (b) {
-                                        const int l = __ffs(b) - 1;
-                                        last_end = p + 16 * l + __ffs(__shfl_sync(0xffffffffu, m, l)) - 1;
-                                        break;
-                                    }
-                                }
+                                // longer than the ring: its fields are read from global memory, up to its end
                                 e = 0xffffu;
                             } else {
                                 step = true;
@@ -2320,13 +2314,11 @@ GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s)
               "                                    keep = ral_keep(P, tx, " << (delims ? "W.db" : "(const ral_u32*)0") << ", s, z, ls, rf);\n"
               "                                    if (pass == 0) refused += rf;\n                                }\n";
     os << R"RALK(                            } else {
-                                ral_i64 n = x != 0xffffu ? (ral_i64)(x - s) : last_end - (base + s);
-                                if (ls[n - 1] == '\r') --n;
-                                keep = n > 0;
+                                const ral_u32 n = x != 0xffffu ? x - s : 0xffffu;
+                                keep = n > 1u || ls[0] != '\r';
 )RALK";
     if (pred)
-        os << "                                if (keep) {\n                                    const ral_u32 r = ral_keep_long(P, ls, n, "
-           << (delims ? "(char)(P.s[6] & 0xffu)" : "(char)0") << ");\n"
+        os << "                                if (keep) {\n                                    const ral_u32 r = ral_keep_long(P, ls, n);\n"
               "                                    keep = (r & 1u) != 0u;\n"
               "                                    if (pass == 0) refused += r >> 1;\n                                }\n";
     os << R"RALK(                            }
@@ -2405,9 +2397,9 @@ GeneratedKernel generate_text_rows_kernel(const TextScanSpec& t, const Shape& s)
         text_slow_vars(std::to_string(q), isf, slow_vars, slow_call, slow_copy);
         args += std::string(", ") + (isf ? "double& x" : "ral_i64& x") + std::to_string(q) + ", ral_u32& w" + std::to_string(q);
     }
-    os << "static __device__ __noinline__ void ral_line_slow(const char* ls, ral_i64 n, char delim, ral_u32& refused" << args
+    os << "static __device__ __noinline__ void ral_line_slow(const RalParams& P, const char* ls, ral_i64 n, ral_u32& refused" << args
        << ") {\n";
-    os << "    ral_i64 fs[" << parts.f2.size() << "], fe[" << parts.f2.size() << "];\n    ral_fields_slow(ls, n, delim, fs, fe);\n";
+    os << "    ral_i64 fs[" << parts.f2.size() << "], fe[" << parts.f2.size() << "];\n" << text_long_end() << "    ral_fields_slow(ls, n, (char)(P.s[6] & 0xffu), (char)(P.s[6] >> 8), fs, fe);\n";
     for (int q = 0; q < NP; q++)
         emit_text_parse(os, "    ", t.dtypes[q], std::to_string(text_slot_of(parts.f2, t.file_cols[q])), "x" + std::to_string(q),
                         "w" + std::to_string(q), false);
@@ -2443,14 +2435,9 @@ GeneratedKernel generate_text_rows_kernel(const TextScanSpec& t, const Shape& s)
         const ral_i64 g = (ral_i64)(ent & 0xffffffffffffull);
         ral_i64 n = (ral_i64)(ent >> 48);
         const int m = (int)(kept - k0 < 32u ? kept - k0 : 32u);
-        const bool lng = n == 65535;
-        if (act && lng) {
-            n = 0;
-            while (g + n < hi && A[g + n] != term) ++n;
-        }
         const ral_i64 a0 = __shfl_sync(0xffffffffu, g, 0) & ~15ll;
         const ral_i64 zl = __shfl_sync(0xffffffffu, g + n, m - 1);
-        const bool any_long = __any_sync(0xffffffffu, act && lng);
+        const bool any_long = __any_sync(0xffffffffu, n == 65535);
         ral_u32 s = 16u;
         bool in = true;
         __syncwarp();
@@ -2487,15 +2474,15 @@ GeneratedKernel generate_text_rows_kernel(const TextScanSpec& t, const Shape& s)
         os << "        " << (isf ? "double x" : "ral_i64 x") << q << " = 0;\n        ral_u32 w" << q << " = 0u;\n";
     }
     os << "        if (act) {\n";
-    os << "            if ((in ? ral_txv_byte<RAL_TXM>(tx, s + (ral_u32)n - 1u) : (ral_u32)(unsigned char)ls[n - 1]) == '\\r') --n;\n";
     os << "            if (in) {\n";
+    os << "                if (ral_txv_byte<RAL_TXM>(tx, s + (ral_u32)n - 1u) == '\\r') --n;\n";
     os << "                ral_u32 fs[" << parts.f2.size() << "], fe[" << parts.f2.size()
        << "];\n                ral_fields(db, s, s + (ral_u32)n, fs, fe);\n";
     for (int q = 0; q < NP; q++)
         emit_text_parse(os, "                ", t.dtypes[q], std::to_string(text_slot_of(parts.f2, t.file_cols[q])),
                         "x" + std::to_string(q), "w" + std::to_string(q), true);
     os << "            } else {\n                ral_u32 rf = 0u;\n                " << slow_vars
-       << "\n                ral_line_slow(ls, n, (char)(P.s[6] & 0xffu), rf" << slow_call << ");\n                " << slow_copy
+       << "\n                ral_line_slow(P, ls, n, rf" << slow_call << ");\n                " << slow_copy
        << "refused += rf;\n            }\n        }\n";
     os << "        const ral_u64 b = k0 + obase;\n";
     for (int q = 0; q < NP; q++) {
