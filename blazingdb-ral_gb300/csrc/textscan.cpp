@@ -63,16 +63,22 @@ struct LineIndex {
     explicit LineIndex(cudaStream_t st) : ends(st) {}
 };
 
-int build_line_index(const char* data, int64_t n, char term, cudaStream_t st, LineIndex& li) {
-    if (n <= 0) return kSuccess;
+// Enqueues the count of data[0, n)'s terminators before each of its tiles, and of all of them after the last.
+int term_offsets(const char* data, int64_t n, char term, cudaStream_t st, StreamBuffer& offsets) {
     const int64_t tiles = text_tiles(n);
-    StreamBuffer counts(st), offsets(st);
+    StreamBuffer counts(st);
     if (int e = counts.alloc((size_t)tiles * 4)) return e;
     if (int e = offsets.alloc((size_t)(tiles + 1) * 8)) return e;
     if (int e = check_cuda(launch_text_term_counts(data, n, term, (uint32_t*)counts.p, st), "line terminators")) return e;
-    if (int e = check_cuda(launch_exclusive_scan_u32((const uint32_t*)counts.p, tiles, (unsigned long long*)offsets.p, st),
-                           "line terminator scan"))
-        return e;
+    return check_cuda(launch_exclusive_scan_u32((const uint32_t*)counts.p, tiles, (unsigned long long*)offsets.p, st),
+                      "line terminator scan");
+}
+
+int build_line_index(const char* data, int64_t n, char term, cudaStream_t st, LineIndex& li) {
+    if (n <= 0) return kSuccess;
+    const int64_t tiles = text_tiles(n);
+    StreamBuffer offsets(st);
+    if (int e = term_offsets(data, n, term, st, offsets)) return e;
     // the terminator count and the last byte decide the line count and the index's size
     thread_local unsigned long long* h = nullptr;
     if (!h && check_cuda(cudaMallocHost((void**)&h, 16), "cudaMallocHost")) return kCudaError;
@@ -97,14 +103,8 @@ int skip_lines(const char* data, int64_t n, char term, int64_t lines, unsigned l
     constexpr int64_t kFew = 16;
     if (lines <= kFew)
         return check_cuda(launch_text_skip(data, n, term, lines, nullptr, out, st), "skipped lines");
-    const int64_t tiles = text_tiles(n);
-    StreamBuffer counts(st), offsets(st);
-    if (int e = counts.alloc((size_t)tiles * 4)) return e;
-    if (int e = offsets.alloc((size_t)(tiles + 1) * 8)) return e;
-    if (int e = check_cuda(launch_text_term_counts(data, n, term, (uint32_t*)counts.p, st), "line terminators")) return e;
-    if (int e = check_cuda(launch_exclusive_scan_u32((const uint32_t*)counts.p, tiles, (unsigned long long*)offsets.p, st),
-                           "line terminator scan"))
-        return e;
+    StreamBuffer offsets(st);
+    if (int e = term_offsets(data, n, term, st, offsets)) return e;
     return check_cuda(launch_text_skip(data, n, term, lines, (const unsigned long long*)offsets.p, out, st), "skipped lines");
 }
 
@@ -291,6 +291,26 @@ int64_t range_bytes(int64_t n, int64_t cap) {
     return std::max<int64_t>(1024, std::min({spread, kept, kTextScanRangeBytes}));
 }
 
+// The kept-line list takes 8 bytes a row that the outputs hold; where that is more than this and than the text
+// itself, its lines are counted first and the list holds no more.  That also keeps the ranges long: 20M lines
+// of 62 bytes into outputs of 200M rows take 0.98 ms, 1.60 uncounted.  A capacity that was counted
+// (text_scan_rows) asks for such a list only for lines of under 8 bytes, where the count is in vain: 40M lines of 4 bytes
+// 0.67 ms, 0.58 uncounted.  With room for up to an eighth of the text's bytes (150M rows: 1.20 ms) nothing is counted.
+constexpr int64_t kListBytes = 64 << 20;
+
+// Lines of data[0, n), one more where the last has its terminator.  Synchronous on st.
+int count_lines(const char* data, int64_t n, char term, cudaStream_t st, int64_t* lines) {
+    StreamBuffer offsets(st);
+    if (int e = term_offsets(data, n, term, st, offsets)) return e;
+    unsigned long long h = 0;
+    if (int e = check_cuda(cudaMemcpyAsync(&h, (unsigned long long*)offsets.p + text_tiles(n), 8, cudaMemcpyDeviceToHost, st),
+                           "cudaMemcpyAsync"))
+        return e;
+    if (int e = check_cuda(cudaStreamSynchronize(st), "line terminators")) return e;
+    *lines = (int64_t)h + 1;
+    return kSuccess;
+}
+
 // The lines of data[0, n) (device memory) that start at or after byte `from` (where a line starts),
 // less the first skip_rows of them: the kept rows go to rows row0 .. of the outputs (whose masks are
 // zeroed), at most cap of them; adds the rows kept and each output's valid rows to kept / valid.
@@ -301,12 +321,17 @@ int scan_piece(const PreparedScan& ps, const char* data, int64_t n, char delim, 
     if (n <= from) return check_cuda(launch_zero_list(zero, st), "text scan masks");
     const ParamLayout& L = ps.gk.layout;
     const int64_t head = (int64_t)((uintptr_t)data & 15);
-    const int64_t rb = range_bytes(n - from, cap);
-    const int64_t ranges = (head + n + rb - 1) / rb;
     const int64_t header = text_scan_header(NP);
     cap = std::max<int64_t>(cap, 0);
     // a kept line has at least one byte and, but for the last, a terminator
-    const int64_t listed = std::min(cap, (n - from + 1) / 2);
+    int64_t listed = std::min(cap, (n - from + 1) / 2);
+    if (listed * 8 > std::max(kListBytes, n - from)) {
+        int64_t lines = 0;
+        if (int e = count_lines(data + from, n - from, term, st, &lines)) return e;
+        listed = std::min(listed, lines);
+    }
+    const int64_t rb = range_bytes(n - from, listed);
+    const int64_t ranges = (head + n + rb - 1) / rb;
     StreamBuffer scratch(st), list(st);
     if (int e = scratch.alloc((size_t)(header + ranges) * 8)) return e;
     if (int e = list.alloc((size_t)listed * 8)) return e;
