@@ -54,30 +54,83 @@ int64_t gather_records_least() {
     return v > 0 ? (int64_t)v : (int64_t)24 << 20;
 }
 
-// launch_gather_columns, or by way of row records (gather_records.cu) where that saves more random accesses
-// than laying the records out costs: two columns or more, whose records are at least half full (8 of 16
-// bytes), and an index that reads a good part of the table.  Whether the index is scattered is found on the device (a flag that the kernels of both ways read), so no
-// synchronisation is added.
-int gather_columns(GatherColumnsParams& p, cudaStream_t st) {
+// The groups of p's columns where row records save more random accesses than laying them out costs (two columns
+// or more, an index that reads a good part of a table of some size), their records in at most `most` bytes; none
+// otherwise.  That the index is scattered, the other condition, is found on the device.
+int record_groups(const GatherColumnsParams& p, int64_t most, GatherGroup* groups, int64_t* bytes) {
     int64_t row = 0;
     for (int c = 0; c < p.num_columns; c++) row += p.col[c].width;
-    const bool records = p.num_columns > 1 && row >= 8 && p.n_out >= kGatherProbeRows && p.n_out >= p.n_in / 4 && p.n_in > 0 &&
-                         p.n_in * row >= gather_records_least();
-    void* scratch = nullptr;
-    if (records) {
-        cudaMemPool_t pool = nullptr;
-        if (int e = scratch_pool(&pool)) return e;
-        if (cudaMallocFromPoolAsync(&scratch, gather_records_bytes(p), pool, st) != cudaSuccess) {
-            cudaGetLastError();  // no room for the records: straight from the columns
-            scratch = nullptr;
+    *bytes = 0;
+    if (p.num_columns < 2 || row < 8 || p.n_out < kGatherProbeRows || p.n_out < p.n_in / 4 || p.n_in <= 0 ||
+        p.n_in * row < gather_records_least())
+        return 0;
+    const int n = gather_groups(p, most, groups, bytes);
+    return *bytes > 0 ? n : 0;
+}
+
+// The most that a call's records take: what the scratch pool keeps between calls, or, given back when the call
+// ends, a quarter of the device memory that is free.  300M rows of six columns in records of 32 bytes (9.6 GB) take
+// 13.4 ms; in two passes of narrower records that stay within what is kept 27.2 ms.
+int64_t gather_records_most(const GatherColumnsParams& p) {
+    const int64_t kept = (int64_t)kScratchPoolKept;
+    if (p.n_in * 64 <= kept) return kept;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return kept;
+    }
+    return std::max(kept, (int64_t)(free_bytes / 4));
+}
+
+// launch_gather_columns, or by way of row records (gather_records.cu) where that is faster.  Up to kGatherAhead
+// bytes of records, half of what the pool keeps, are allocated before it is known whether the index is scattered (a
+// flag that the kernels of both ways read), so that nothing is waited for: the wait is 13 us, of 340 at 8M rows and
+// of 3740 at 100M.  For more the flag comes back first, since a clustered index would leave the memory unused
+// and pay for its mapping (300M rows in order 4.0 ms, 6.3 with 9.6 GB of records allocated for nothing).
+constexpr int64_t kGatherAhead = (int64_t)kScratchPoolKept / 2;
+int gather_columns(GatherColumnsParams& p, cudaStream_t st) {
+    GatherGroup groups[kMaxGatherColumns];
+    int64_t bytes = 0;
+    const int n = record_groups(p, gather_records_most(p), groups, &bytes);
+    if (!n) return check_cuda(launch_gather_columns(p, st), "gather_columns");
+    // the flag, then the records
+    void *flag = nullptr, *records = nullptr;
+    cudaMemPool_t pool = nullptr;
+    if (int e = scratch_pool(&pool)) return e;
+    const bool ahead = bytes <= kGatherAhead;
+    if (cudaMallocFromPoolAsync(&flag, ahead ? 256 + (size_t)bytes : 256, pool, st) != cudaSuccess) {
+        cudaGetLastError();  // no room: straight from the columns
+        return check_cuda(launch_gather_columns(p, st), "gather_columns");
+    }
+    p.scattered = (const int32_t*)flag;
+    int rc = check_cuda(launch_gather_probe(p, (int32_t*)flag, st), "gather_probe");
+    if (!rc && ahead) records = (char*)flag + 256;
+    if (!rc && !ahead) {
+        int32_t scattered = 0;
+        rc = check_cuda(cudaMemcpyAsync(&scattered, flag, sizeof scattered, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+        if (!rc) rc = check_cuda(cudaStreamSynchronize(st), "gather_probe");
+        if (!rc && scattered && cudaMallocFromPoolAsync(&records, (size_t)bytes, pool, st) != cudaSuccess) {
+            cudaGetLastError();
+            records = nullptr;
+        }
+        if (!rc && scattered && !records) p.scattered = nullptr;
+    }
+    if (!rc && records) {
+        rc = check_cuda(launch_gather_records(p, groups, n, records, st), "gather_records");
+        // what no record holds, where the index is scattered
+        for (int g = 0; g < n && !rc; g++) {
+            if (groups[g].record) continue;
+            GatherColumnsParams rest = p;
+            rest.num_columns = groups[g].to - groups[g].from;
+            std::copy(p.col + groups[g].from, p.col + groups[g].to, rest.col);
+            if (rest.valid_counts) rest.valid_counts += groups[g].from;
+            rest.only_scattered = 1;
+            rc = check_cuda(launch_gather_columns(rest, st), "gather_columns");
         }
     }
-    if (!scratch) return check_cuda(launch_gather_columns(p, st), "gather_columns");
-    p.scattered = (const int32_t*)scratch;
-    int rc = check_cuda(launch_gather_probe(p, (int32_t*)scratch, st), "gather_probe");
-    if (!rc) rc = check_cuda(launch_gather_records(p, scratch, st), "gather_records");
     if (!rc) rc = check_cuda(launch_gather_columns(p, st), "gather_columns");
-    cudaFreeAsync(scratch, st);
+    if (records && !ahead) cudaFreeAsync(records, st);
+    cudaFreeAsync(flag, st);
     return rc;
 }
 
@@ -449,6 +502,27 @@ int ral_materialize_columns(const gdf_column* const* inputs, gdf_column* const* 
             outputs[c]->size = (gdf_size_type)n;
             outputs[c]->null_count = outputs[c]->valid ? (gdf_size_type)(n - (int64_t)h[c]) : 0;
         }
+        return (int)kSuccess;
+    });
+}
+
+int ral_debug_gather_plan(const int32_t* widths, const int32_t* masked, int32_t num_columns, int64_t rows_in,
+                          int64_t rows_out, int64_t most_bytes, int32_t* record_bytes, int64_t* scratch_bytes) {
+    return guarded([&] {
+        if (!widths || !masked || !record_bytes || !scratch_bytes || num_columns < 0 || num_columns > kMaxGatherColumns)
+            return set_error(kInvalidArgument, "bad argument");
+        GatherColumnsParams p{};
+        p.num_columns = num_columns;
+        p.n_in = rows_in;
+        p.n_out = rows_out;
+        for (int c = 0; c < num_columns; c++) {
+            uint32_t* const mask = masked[c] ? (uint32_t*)(uintptr_t)256 : nullptr;  // only its presence matters
+            p.col[c] = GatherColumn{nullptr, mask, nullptr, mask, widths[c], 0};
+        }
+        GatherGroup groups[kMaxGatherColumns];
+        const int n = record_groups(p, most_bytes, groups, scratch_bytes);
+        std::fill(record_bytes, record_bytes + num_columns, 0);
+        for (int g = 0; g < n; g++) std::fill(record_bytes + groups[g].from, record_bytes + groups[g].to, groups[g].record);
         return (int)kSuccess;
     });
 }

@@ -251,21 +251,13 @@ __global__ void __launch_bounds__(kThreads, 3) record_gather_kernel(const __grid
         atomicAdd(P.col[threadIdx.x].count, (unsigned long long)s_cnt[threadIdx.x]);
 }
 
-// The next group of columns (from column `from` on) whose record takes at most 64 bytes: their places in
-// P, the record's words, and the column after the group.
-int next_group(const GatherColumnsParams& p, int from, RecordParams& P, int* words) {
-    int bytes = 0, masks = 0, to = from;
-    for (; to < p.num_columns; to++) {
-        const int b = bytes + p.col[to].width, m = masks + (p.col[to].in_valid && p.col[to].out_valid ? 1 : 0);
-        if (b + (m + 7) / 8 > 64) break;
-        bytes = b;
-        masks = m;
-    }
+// A group's columns (of which some may follow in p): their places in the record.
+void place_group(const GatherColumnsParams& p, const GatherGroup& group, RecordParams& P) {
     // widest first, so that every element is aligned; the bits after the last
     int at = 0, bit = 0;
     P.num_columns = 0;
     for (int w = 8; w >= 1; w /= 2)
-        for (int c = from; c < to; c++) {
+        for (int c = group.from; c < group.to; c++) {
             const GatherColumn& g = p.col[c];
             if (g.width != w) continue;
             RecordColumn& r = P.col[P.num_columns++];
@@ -281,9 +273,6 @@ int next_group(const GatherColumnsParams& p, int from, RecordParams& P, int* wor
         }
     P.bits_at = at;
     P.bits_bytes = (bit + 7) / 8;
-    const int size = at + (bit + 7) / 8;
-    *words = size <= 16 ? 4 : size <= 32 ? 8 : 16;
-    return to;
 }
 
 template <int W>
@@ -296,32 +285,46 @@ void group_passes(const RecordParams& P, int grid, cudaStream_t st) {
 
 }  // namespace
 
-// The flag comes first, then the records.
-size_t gather_records_bytes(const GatherColumnsParams& p) {
-    int most = 4;
-    RecordParams P{};
-    for (int c = 0; c < p.num_columns;) {
-        int w = 0;
-        c = next_group(p, c, P, &w);
-        most = std::max(most, w);
+// Columns are taken in order, as many as fit a record; the record is then the smallest that holds them.  Records of
+// 64 bytes are the fewest passes; where the input's rows make that more than `most` bytes, 32 or 16.
+int gather_groups(const GatherColumnsParams& p, int64_t most, GatherGroup* groups, int64_t* bytes) {
+    *bytes = 0;
+    int64_t width = 64;
+    while (width >= 16 && p.n_in * width > most) width /= 2;
+    int n = 0;
+    for (int from = 0; from < p.num_columns; n++) {
+        int size = 0, elements = 0, masks = 0, to = from;
+        for (; to < p.num_columns; to++) {
+            const int e = elements + p.col[to].width, m = masks + (p.col[to].in_valid && p.col[to].out_valid ? 1 : 0);
+            if (to > from && e + (m + 7) / 8 > width) break;
+            elements = e;
+            masks = m;
+            size = e + (m + 7) / 8;
+        }
+        groups[n] = GatherGroup{from, to, size <= 16 ? 16 : size <= 32 ? 32 : 64};
+        // a record of one column, or one less than half full, costs more than the accesses it saves (eight columns
+        // of 8 bytes and a ninth, 8M rows: 565 us straight, 641 with it in records of its own; two of one byte 598, 631)
+        if (to - from < 2 || size < 8 || groups[n].record > width) groups[n].record = 0;
+        *bytes = std::max(*bytes, p.n_in * groups[n].record);
+        from = to;
     }
-    return 256 + (size_t)p.n_in * 4 * most;
+    return n;
 }
 
-cudaError_t launch_gather_records(const GatherColumnsParams& p, void* scratch, cudaStream_t st) {
+cudaError_t launch_gather_records(const GatherColumnsParams& p, const GatherGroup* groups, int n_groups, void* records, cudaStream_t st) {
     RecordParams P{};
     P.idx = p.idx;
     P.idx_width = p.idx_width;
     P.n_in = p.n_in;
     P.n_out = p.n_out;
-    P.scattered = (const int32_t*)scratch;
-    P.records = (uint4*)((char*)scratch + 256);
+    P.scattered = p.scattered;
+    P.records = (uint4*)records;
     const int grid = (int)std::min<int64_t>((int64_t)device_sms() * 8, (std::max(p.n_in, p.n_out) + kThreads - 1) / kThreads);
-    for (int c = 0; c < p.num_columns;) {
-        int words = 0;
-        c = next_group(p, c, P, &words);
-        if (words == 4) group_passes<4>(P, grid, st);
-        else if (words == 8) group_passes<8>(P, grid, st);
+    for (int g = 0; g < n_groups; g++) {
+        if (!groups[g].record) continue;
+        place_group(p, groups[g], P);
+        if (groups[g].record == 16) group_passes<4>(P, grid, st);
+        else if (groups[g].record == 32) group_passes<8>(P, grid, st);
         else group_passes<16>(P, grid, st);
         if (cudaError_t e = cudaGetLastError()) return e;
     }

@@ -206,7 +206,7 @@ __device__ __noinline__ int ral_gather_votes(const GatherColumnsParams& P, int w
 // 48 registers, five resident blocks of 256 threads per SM (a bound of six spills registers in the
 // gather loops).
 __global__ void __launch_bounds__(256, 5) gather_columns_kernel(const __grid_constant__ GatherColumnsParams P) {
-    if (P.scattered && *P.scattered) return;
+    if (P.scattered && (*P.scattered != 0) != (P.only_scattered != 0)) return;
     __shared__ unsigned long long s_cnt[kMaxGatherColumns];
     __shared__ int s_clustered;
     for (int c = threadIdx.x; c < P.num_columns; c += blockDim.x) s_cnt[c] = 0;
@@ -222,8 +222,7 @@ __global__ void __launch_bounds__(256, 5) gather_columns_kernel(const __grid_con
         if (lane == 0) atomicAdd(&s_clustered, votes);
     }
     __syncthreads();
-    const bool row_major =
-        P.scattered || P.num_columns == 1 || P.n_out < 32 * kGatherSamples || 2 * s_clustered >= kGatherSamples;
+    const bool row_major = P.num_columns == 1 || (P.scattered ? P.only_scattered == 0 : P.n_out < 32 * kGatherSamples || 2 * s_clustered >= kGatherSamples);
     const ral_i64 step_rows = 32 * kGatherRowsPerLane;
     const ral_i64 nsteps = (P.n_out + step_rows - 1) / step_rows;
     const ral_i64 gwarp = ((ral_i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;

@@ -40,9 +40,10 @@ struct GatherColumnsParams {
     unsigned long long* valid_counts;  // one counter per column with out_valid (zeroed), or null
     int32_t num_columns;
     int32_t idx_width;  // 1, 2, 4 or 8
-    // optional: nonzero where the index is scattered (launch_gather_probe), and another launch gathers the
-    // columns then
+    // optional: nonzero where the index is scattered (launch_gather_probe); the launch gathers the columns where
+    // that is only_scattered and leaves them to another one otherwise
     const int32_t* scattered;
+    int32_t only_scattered;  // 0 or 1
 };
 
 // out_c[i] = in_c[idx[i]] for every column c, reading each index once; other indices leave
@@ -55,10 +56,16 @@ cudaError_t launch_gather_columns(const GatherColumnsParams& p, cudaStream_t st)
 constexpr int64_t kGatherProbeRows = 2048;
 cudaError_t launch_gather_probe(const GatherColumnsParams& p, int32_t* scattered, cudaStream_t st);
 
-// Every column by way of row records in `scratch` (gather_records.cu), where the int32 flag at its start
-// is nonzero; nothing where it is zero.  p.n_in at least 1.
-size_t gather_records_bytes(const GatherColumnsParams& p);
-cudaError_t launch_gather_records(const GatherColumnsParams& p, void* scratch, cudaStream_t st);
+// Columns [from, to) of p, gathered by way of records of 16, 32 or 64 bytes, or (0) straight from the columns.
+struct GatherGroup {
+    int32_t from, to, record;
+};
+// p's columns in groups (at most kMaxGatherColumns); *bytes is what the records of the largest take, at most
+// `most`.
+int gather_groups(const GatherColumnsParams& p, int64_t most, GatherGroup* groups, int64_t* bytes);
+// The groups that go by way of records, one after the other in `records` (16-byte aligned), where *p.scattered is
+// nonzero; nothing where it is zero.  p.n_in at least 1.
+cudaError_t launch_gather_records(const GatherColumnsParams& p, const GatherGroup* groups, int n_groups, void* records, cudaStream_t st);
 
 // ---- line index of a delimited text buffer (the text scan) ---------------------------------
 

@@ -54,6 +54,8 @@ _SIGS = {
     "ral_process_aggregate": (C.c_int, [C.c_void_p, C.c_int32, C.c_char_p, C.POINTER(GdfScalar), C.c_int32,
                                         C.POINTER(C.c_int32)]),
     "ral_debug_call_timing": (C.c_int, [C.c_int32, C.c_int32, C.POINTER(C.c_int64), C.POINTER(C.c_double)]),
+    "ral_debug_gather_plan": (C.c_int, [I32P, I32P, C.c_int32, C.c_int64, C.c_int64, C.c_int64, I32P,
+                                        C.POINTER(C.c_int64)]),
     "ral_debug_filter_grid_launches": (C.c_int, [C.POINTER(C.c_int64)]),
     "ral_text_scan_rows": (C.c_int, [C.c_void_p, C.c_int64, C.c_char, C.c_int32, C.POINTER(C.c_int64)]),
     "ral_text_scan_filter": (C.c_int, [C.c_void_p, C.c_int64, C.c_char, C.c_char, C.c_int32, I32P, C.c_int32, I32P,
@@ -601,6 +603,14 @@ def filter_grid_launches() -> int:
     v = C.c_int64(0)
     _check(lib().ral_debug_filter_grid_launches(C.byref(v)))
     return v.value
+
+
+def debug_gather_plan(widths, masked, rows_in: int, rows_out: int, most: int = 8 << 30) -> Tuple[List[int], int]:
+    """The row record's bytes that each column travels in (0: gathered straight from the column) and the
+    device memory that the records take, of at most `most` bytes."""
+    w, m, rec, total = _i32(widths), _i32(masked), _i32([0] * len(widths)), C.c_int64(0)
+    _check(lib().ral_debug_gather_plan(_p32(w), _p32(m), len(w), rows_in, rows_out, most, _p32(rec), C.byref(total)))
+    return [int(x) for x in rec], total.value
 
 
 class Category:

@@ -58,6 +58,13 @@ int ral_debug_call_timing(int32_t enable, int32_t reset, int64_t *calls, double 
  * all fit on the device: one cooperative launch, a grid barrier in place of the look-back). */
 int ral_debug_filter_grid_launches(int64_t *launches);
 
+/* How ral_materialize_columns gathers columns of these widths (masked[c] != 0: with masks on both sides) by a
+ * scattered index: record_bytes[c] receives the size of the row record column c travels in, 0 where it is
+ * gathered straight from the column, and *scratch_bytes the device memory that the records take, of at most
+ * most_bytes.  Needs no GPU. */
+int ral_debug_gather_plan(const int32_t *widths, const int32_t *masked, int32_t num_columns, int64_t rows_in,
+                          int64_t rows_out, int64_t most_bytes, int32_t *record_bytes, int64_t *scratch_bytes);
+
 /* Generated source of the text scan kernel for a file schema, projections and filter (NULL: none),
  * with an NVRTC-only compile when compile != 0 (log_out gets the ptxas log); needs no GPU. */
 int ral_debug_text_scan_source(const int32_t *file_dtypes, int32_t n_file_columns, const int32_t *projections,
