@@ -881,6 +881,10 @@ int ral_autotune_program(gdf_column* const* output_columns, int32_t num_outputs,
     });
 }
 
+int ral_trim_scratch(void) {
+    return guarded([&] { return trim_scratch_pool(); });
+}
+
 int64_t ral_kernel_launches(void) { return (int64_t)launch_count(); }
 
 int ral_jit_stats(int64_t* compiles, int64_t* disk_hits, int64_t* memory_hits, double* compile_ms) {

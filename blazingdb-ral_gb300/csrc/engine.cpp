@@ -163,6 +163,12 @@ int scratch_pool(cudaMemPool_t* out) {
     return kSuccess;
 }
 
+int trim_scratch_pool() {
+    cudaMemPool_t pool = nullptr;
+    if (int e = scratch_pool(&pool)) return e;
+    return check_cuda(cudaMemPoolTrimTo(pool, 0), "cudaMemPoolTrimTo");
+}
+
 int scratch_alloc(void** out, size_t bytes, cudaStream_t st) {
     cudaMemPool_t pool = nullptr;
     if (int e = scratch_pool(&pool)) return e;

@@ -94,6 +94,8 @@ void keep_pool_memory();
 // calls have freed it keeps at most kScratchPoolKept bytes at a synchronisation.
 constexpr uint64_t kScratchPoolKept = (uint64_t)8 << 30;
 int scratch_pool(cudaMemPool_t* out);
+// What calls have freed to that pool, given back to the device.
+int trim_scratch_pool();
 // Stream-ordered scratch of one call from that pool (freed with cudaFreeAsync).  The device's default
 // pool keeps nothing at a synchronisation unless the process asks it to, so that an allocation there
 // maps memory again on every call: about 130 us for eight bytes.

@@ -54,6 +54,7 @@ _SIGS = {
     "ral_process_aggregate": (C.c_int, [C.c_void_p, C.c_int32, C.c_char_p, C.POINTER(GdfScalar), C.c_int32,
                                         C.POINTER(C.c_int32)]),
     "ral_debug_call_timing": (C.c_int, [C.c_int32, C.c_int32, C.POINTER(C.c_int64), C.POINTER(C.c_double)]),
+    "ral_trim_scratch": (C.c_int, []),
     "ral_debug_gather_plan": (C.c_int, [I32P, I32P, C.c_int32, C.c_int64, C.c_int64, C.c_int64, I32P,
                                         C.POINTER(C.c_int64)]),
     "ral_debug_filter_grid_launches": (C.c_int, [C.POINTER(C.c_int64)]),
@@ -596,6 +597,11 @@ def call_timing(enable: bool = True, reset: bool = False) -> dict:
     _check(lib().ral_debug_call_timing(1 if enable else 0, 1 if reset else 0, C.byref(calls), us))
     return {"calls": calls.value, "host_prepare_us": us[0], "enqueue_us": us[1], "wait_us": us[2],
             "kernel_device_us": us[3]}
+
+
+def trim_scratch() -> None:
+    """Gives the unused memory of the library's scratch pool on the current device back."""
+    _check(lib().ral_trim_scratch())
 
 
 def filter_grid_launches() -> int:

@@ -392,6 +392,10 @@ int ral_autotune_program(gdf_column *const *output_columns, int32_t num_outputs,
                          const gdf_scalar *right_scalars, int32_t *best_slices, int32_t *best_unroll,
                          int32_t *best_soft_fp, double *best_ms);
 
+/* Gives the unused memory of the library's scratch pool on the current device back to the device (calls keep
+ * at most 8 GB there for the next one).  Safe beside calls of other threads: what they use stays. */
+int ral_trim_scratch(void);
+
 /* Kernels launched by this library since load (all entry points). */
 int64_t ral_kernel_launches(void);
 
