@@ -74,8 +74,10 @@ bool reads_host_pages() {
     return v != 0;
 }
 
-// Whether eight pages spread over file[0, n) are all in memory (3 us).  A mapped file that has not been read
-// yet would come in by a fault of the device per page: it is copied in, which reads it in order.
+// Whether eight pages spread over file[0, n) are all in memory (3 us): a sample, taken before the call reads
+// anything of the file itself (its footer and page headers lie all over it).  A mapped file that has not been read
+// yet would come in by a fault of the device per page: it is copied in, which reads it in order.  A file that is
+// partly in memory can pass; its other pages then come in by such faults, with the same result.
 bool resident(const uint8_t* file, int64_t n) {
     const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
     for (int64_t k = 0; k < 8; k++) {
@@ -88,9 +90,10 @@ bool resident(const uint8_t* file, int64_t n) {
 
 // The address kernels read file[0, n) at, or null where the chunks are to be copied in: page-locked (or
 // mapped) host memory of this process, and, where the device reads them at the link's rate too, ordinary
-// pages.  A copy from those returns when it is done, so nothing overlapped it: 700,001 rows of dictionary
-// pages with nulls 260 us copied, 226 in place; 6M rows of PLAIN pages 1365 and 1021; 10,000 rows 108
-// and 100.  Both ends are checked: a registered range covers the whole buffer.
+// pages.  A copy from those returns when it is done, so nothing overlaps it.  Buffers that the device has not read
+// before, in place against copied (and when they are scanned again): 10,000 rows 122 and 129 us (105, 109),
+// 700,001 rows of dictionary pages with nulls 209 and 276 (185, 236), 6M rows of PLAIN pages 1038 and 1385 (927,
+// 1203).  Both ends are checked: a registered range covers the whole buffer.
 const uint8_t* device_view(const uint8_t* file, int64_t n) {
     if (std::getenv("RAL_PARQUET_STAGED")) return nullptr;  // always copy the chunks in
     cudaPointerAttributes a{}, b{};
@@ -332,6 +335,8 @@ int parquet_scan_filter(const uint8_t* file, int64_t n, const int32_t* projectio
                         gdf_column* const* outs, gdf_size_type* n_out) {
     if (!projections || n_proj <= 0 || !outs || !n_out) return set_error(kInvalidArgument, "bad argument");
     if (n_proj > kParquetMaxColumns) return set_error(kUnsupported, "more than 64 projected columns");
+    if (!file || n <= 0) return set_error(kInvalidArgument, "bad argument");
+    const uint8_t* direct = device_view(file, n);
     pq::FileMeta meta;
     if (int e = read_meta(file, n, meta)) return e;
     const int64_t rows = meta.num_rows;
@@ -366,7 +371,6 @@ int parquet_scan_filter(const uint8_t* file, int64_t n, const int32_t* projectio
     // it is copied in, chunk by chunk.  Chunks with dictionary-encoded pages that are not decompressed are
     // copied to device memory by a kernel even then: dictionaries are looked up at random, and the walk of
     // the indices' run headers waits for every read (runs of 504 values: 325 us copied, 468 in place).  Snappy pages are decompressed into the unpack buffer.
-    const uint8_t* direct = device_view(file, n);
     std::vector<int64_t> copied(plan.chunks.size(), -1);  // in place: where a chunk that is copied goes
     int64_t file_bytes = direct ? 0 : plan.packed;
     if (direct) {
