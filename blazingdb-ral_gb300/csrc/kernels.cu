@@ -1476,7 +1476,7 @@ cudaError_t launch_copy_list(const CopyList& list, cudaStream_t st) {
     for (int k = 0; k < list.n; k++) most = std::max(most, list.job[k].bytes);
     if (most <= 0) return cudaSuccess;
     // 4 of the 16-byte words a thread, up to the device's threads for all jobs together
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((most + 16383) / 16384, (152 * 8 + list.n - 1) / list.n));
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((most + 16383) / 16384, ((int64_t)device_sms() * 8 + list.n - 1) / list.n));
     copy_list_kernel<<<dim3((unsigned)blocks, (unsigned)list.n), 256, 0, st>>>(list);
     note_launch();
     return cudaGetLastError();
@@ -1506,7 +1506,7 @@ cudaError_t launch_zero_list(const ZeroList& list, cudaStream_t st) {
     int64_t most = 0;
     for (int k = 0; k < list.n; k++) most = std::max(most, list.words[k]);
     // 4 of the 16-byte words a thread, up to the device's threads for all ranges together
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((most + 4095) / 4096, (152 * 8 + list.n - 1) / list.n));
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((most + 4095) / 4096, ((int64_t)device_sms() * 8 + list.n - 1) / list.n));
     zero_list_kernel<<<dim3((unsigned)blocks, (unsigned)list.n), 256, 0, st>>>(list);
     note_launch();
     return cudaGetLastError();
