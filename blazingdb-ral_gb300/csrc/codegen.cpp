@@ -2069,8 +2069,8 @@ void emit_text_params(std::ostream& os, bool delims) {
 // lines' count goes through the look-back while the warp scans its next range; their positions wait in
 // shared memory, or, where a range keeps more of them than fit, the range is read a second time.
 //
-// Bound: instruction issue (70% of the slots, the ALU pipe as busy), about 1000 instructions per 32 lines for
-// TPC-H Q6's three fields and conditions, 510 of them for finding the lines.  The text is read once and no
+// Bound: instruction issue (67% of the slots, the ALU pipe 65%), 1080 instructions per 32 lines of 66 bytes for
+// TPC-H Q6's three fields and conditions, half of them for finding the lines.  The text is read once and no
 // line index is written: 20M lines of 62 bytes take 0.80 ms (1.6 TB/s of text), against 2.96 ms for a line
 // index of three kernels and then a walk of every line byte by byte.
 GeneratedKernel generate_text_scan_kernel(const TextScanSpec& t, const Shape& s) {

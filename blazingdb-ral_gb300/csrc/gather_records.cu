@@ -8,7 +8,7 @@
 // Six columns of 100M rows (29 bytes and six validity bits a row) by a permutation: 13.6 ms straight from
 // the columns, 3.72 ms here; 30M rows 3.16 / 1.16, 4M rows 0.236 / 0.180, 1M rows 0.083 / 0.072 ms (below
 // that the two extra launches cost more than the accesses saved).  Of 30M rows' 1.16 ms the pack takes
-// 0.3 (60 bytes a row streamed) and the gather 0.8: 40 G random records a second, a rate that the card
+// 0.33 (60 bytes a row streamed) and the gather 0.70: 43 G random records a second, a rate that the card
 // does not exceed for 8-byte or 32-byte accesses, 64 or 128 bytes fetched, alike.
 #include <cuda_runtime.h>
 
@@ -178,7 +178,7 @@ __device__ __forceinline__ ral_u32 unpack_column(const RecordParams& P, const Re
 }
 
 // 16 bytes of a record.  The record's 64-byte DRAM access is all that is wanted: without the qualifier a
-// miss fetches the 128 bytes around it (30M random 32-byte records read 3.8 GB; 2.1 GB with it).
+// miss fetches the 128 bytes around it (30M random 32-byte records read 3.7 GB in 737 us; 2.0 GB in 695 with it).
 __device__ __forceinline__ uint4 load_part(const uint4* p) {
     uint4 v;
     asm("ld.global.L2::64B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));

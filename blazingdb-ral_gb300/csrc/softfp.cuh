@@ -804,7 +804,7 @@ RAL_SF_CALL double ral_sf_sincos_far(double x, bool want_cos) {
 // About 200 integer instructions against some 20 FP64 ones of the library's function, each of which takes the
 // FP64 pipe as long as 64 integer instructions take the SM: a projection of SIN over 50M rows 570 us (1798
 // with the library's), of SIN(COS(SIN(x * y))) 1409 (5255), 256 programs over tables of up to 1M rows
-// 7.2 ms (16.2).
+// 6.5 ms (16.2).
 RAL_SF double ral_sf_sincos(double x, bool want_cos) {
     const unsigned long long X = ral_sf_obits(x);
     const int ex = (int)((X >> 52) & 0x7ff);
