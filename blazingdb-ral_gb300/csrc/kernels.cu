@@ -1023,7 +1023,9 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const __grid_consta
         return;
     }
     // PLAIN values, or a dictionary's entries through the present rows' indices
-    const int64_t nvals = pg.dict_count > 0 ? (int64_t)0x7fffffffffffffffll : (pg.data_bytes - lo) / w;
+    // the page's values, or its rows' places in the indices: where its levels did not read, the items' first
+    // values are not their ranks in the page
+    const int64_t nvals = pg.dict_count > 0 ? (int64_t)pg.rows : (pg.data_bytes - lo) / w;
     const uint8_t* const dict = (const uint8_t*)pg.dict;
     const uint32_t* const ix = P.idx + pg.idx0;
     // this item's validity words, page-relative (rows of the next page masked off)
@@ -1068,7 +1070,7 @@ __global__ void __launch_bounds__(256) parquet_values_kernel(const __grid_consta
         if (pg.dict_count > 0) {
             uint32_t k[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) k[u] = vi[u] >= 0 ? ix[vi[u]] : 0xffffffffu;
+            for (int u = 0; u < 4; ++u) k[u] = vi[u] >= 0 && vi[u] < nvals ? ix[vi[u]] : 0xffffffffu;
 #pragma unroll
             for (int u = 0; u < 4; ++u) x[u] = k[u] < (uint32_t)pg.dict_count ? ral_pq_value(dict, k[u], w) : 0ull;
         } else {
