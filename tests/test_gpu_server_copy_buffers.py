@@ -66,3 +66,25 @@ def test_page_locked_host_buffers_take_the_copy(served, host):
     arr, structs = _colarray(outs)
     _check(lib().ral_server_copy_result(srv._h, rid, arr, 2))
     _check_outs(outs, structs, exp)
+
+
+def test_buffers_of_one_allocation_and_of_several(served):
+    """Columns in slices of one allocation, in allocations of their own, and at an allocation's very end."""
+    srv, rid, n, exp = served
+    one = torch.full((1 << 20,), 0x5A, dtype=torch.uint8, device="cuda")
+    at = one.numel()
+    outs = []
+    for k, e in enumerate(exp):
+        w = D.WIDTH[e.dtype]
+        at = (at - n * w) // w * w if k else at - n * w
+        data = one[at:at + n * w].view(torch.int32 if w == 4 else torch.int64)
+        valid = torch.zeros((n + 7) // 8 + 64, dtype=torch.uint8, device="cuda")
+        outs.append(R.Column(data, valid, e.dtype, size=n))
+    arr, structs = _colarray(outs)
+    _check(lib().ral_server_copy_result(srv._h, rid, arr, 2))
+    for o, st, e in zip(outs, structs, exp):
+        ev = e.valid_bools()
+        assert st.size == n and st.null_count == e.null_count
+        np.testing.assert_array_equal(np.unpackbits(o.valid.cpu().numpy(), bitorder="little")[:n].astype(bool), ev)
+        np.testing.assert_array_equal(o.data.cpu().numpy()[ev], e.to_numpy().view(o.data.cpu().numpy().dtype)[ev])
+    assert bool((one[:at] == 0x5A).all())
